@@ -109,7 +109,7 @@ void launch_rows_class(const uint4* items, int count, int rows_per_item, const B
         k2p_rows<LOGC, KP, TableRowWork><<<ctas, k2p_threads(LOGC, KP), smem, st>>>(w, B.d_pc, B.d_tw_fwd,
                                                                                     B.d_tw_inv, 4, err);
     } else {
-        const size_t smem = size_t(rows_per_item) * 24 * C;
+        const size_t smem = size_t(rows_per_item) * 12 * C;
         if (smem > 48 * 1024)
             cuda_check(cudaFuncSetAttribute(k2_rows_items<LOGC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             int(smem)),

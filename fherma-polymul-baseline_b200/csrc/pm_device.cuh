@@ -165,14 +165,15 @@ __device__ __forceinline__ void pass_load(uint32_t (&v)[1 << LV], const uint32_t
     }
 }
 
-template <int K, bool WL, int LV = 3>
+// the first U of a pass's K stages (U < K: the closing pass, whose last two stages are deferred)
+template <int K, bool WL, int LV = 3, int U = K>
 __device__ __forceinline__ void pass_forward(uint32_t (&va)[1 << LV], uint32_t (&vb)[1 << LV], int tid, int T, int s0,
                                              int logd, const uint2* tw, uint32_t p, uint32_t two_p) {
 #pragma unroll
     for (int m = 0; m < ((1 << LV) >> K); ++m) {
         const int blk = pass_gid<K, WL, LV>(tid, T, m) >> logd;
 #pragma unroll
-        for (int u = 0; u < K; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int h = 1 << (K - 1 - u);
             const uint2* tws = tw + ((1 << (s0 + u)) + (blk << u));
 #pragma unroll
@@ -186,14 +187,14 @@ __device__ __forceinline__ void pass_forward(uint32_t (&va)[1 << LV], uint32_t (
     }
 }
 
-template <int K, bool WL, int LV = 3>
+template <int K, bool WL, int LV = 3, int U = K>
 __device__ __forceinline__ void pass_inverse(uint32_t (&v)[1 << LV], int tid, int T, int s0, int logd, const uint2* tw,
                                              uint32_t p, uint32_t two_p) {
 #pragma unroll
     for (int m = 0; m < ((1 << LV) >> K); ++m) {
         const int blk = pass_gid<K, WL, LV>(tid, T, m) >> logd;
 #pragma unroll
-        for (int u = K - 1; u >= 0; --u) {
+        for (int u = U - 1; u >= 0; --u) {
             const int h = 1 << (K - 1 - u);
             const uint2* tws = tw + ((1 << (s0 + u)) + (blk << u));
 #pragma unroll
@@ -213,10 +214,28 @@ __device__ __forceinline__ void exchange_sync(bool warp_local) {
         __syncthreads();
 }
 
-// The forward row stages of a and b, the pointwise product and the inverse row
-// stages of one row, starting from the values a thread holds for the first pass
-// (pass_index<KP, false, LV> with s0 = 0) and ending with the product in the
-// same places.  sa, sb: 2C words of exchange space; stf, sti: the row's twiddles.
+// How a row's LOGC - 2 stages (the last two are deferred, see quad_product) are split into
+// passes: NP full passes of KP stages, a pass of MID stages at stride 4 where the rest does
+// not fit the closing pass, and the closing pass, whose groups are runs of 4 * 2^CL values: CL
+// stages, then the products of 4-value polynomials.
+template <int LOGC, int KP, int LV>
+struct RowPlan {
+    static constexpr int S = LOGC - kDeferred;
+    static constexpr int NP = S / KP;
+    static constexpr int REM = S - NP * KP;
+    static constexpr int MID = REM > LV - kDeferred ? REM : 0;
+    static constexpr int CL = MID ? 0 : REM;
+    static constexpr int KC = CL + kDeferred;  // the closing pass's layout: groups of 2^KC values at stride 1
+    static constexpr int K0 = NP ? KP : (MID ? MID : KC);  // the first pass's layout
+    static constexpr int LOGD0 = LOGC - K0;
+    static_assert(LOGC >= 3 && KP <= LV && LV >= 3, "rows of at least 8 values, passes that fit a thread");
+};
+
+// The forward row stages of a and b, the products of the row's 4-value polynomials and the
+// inverse row stages, starting from the values a thread holds for the first pass
+// (pass_index<K0, false, LV> at stride 2^LOGD0 of its RowPlan) and ending with the product in
+// the same places.  sa, sb: 2C words of exchange space; stf, sti: the row's twiddles, C/4
+// entries each.
 // Every exchange stores a thread's values back to the very words that thread
 // loaded in the pass (so no barrier is needed before the store), then meets the
 // others before the next pass loads its own layout.  after_last_load() runs on
@@ -230,13 +249,15 @@ template <int LOGC, int KP, class Hook = NoHook, int LV = 3>
 __device__ __forceinline__ void row_transform(uint32_t (&va)[1 << LV], uint32_t (&vb)[1 << LV], uint32_t* sa,
                                               uint32_t* sb, const uint2* stf, const uint2* sti, int tid,
                                               const PrimeConst& pc, Hook after_last_load = Hook{}) {
+    using Plan = RowPlan<LOGC, KP, LV>;
     constexpr int C = 1 << LOGC;
     constexpr int T = C >> LV;
-    constexpr int NP = LOGC / KP;   // full passes
-    constexpr int REM = LOGC % KP;  // stages of the closing pass
+    constexpr int NP = Plan::NP, MID = Plan::MID, CL = Plan::CL, KC = Plan::KC;
+    constexpr int KM = MID ? MID : 1;  // (unused when there is no such pass)
     constexpr bool WL = KP == LV && T >= 32;
-    constexpr int KR = REM > 0 ? REM : KP;  // closing pass radix (unused when REM = 0)
-    static_assert(KP <= LV, "a pass holds at most V values per group");
+    // layouts that keep a warp inside its own words
+    constexpr bool mid_local = pass_warp_local<KM, WL, LV>(kDeferred), close_local = pass_warp_local<KC, WL, LV>(0);
+    // --- forward ---
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
         const int s0 = KP * q, logd = LOGC - s0 - KP;
@@ -245,34 +266,64 @@ __device__ __forceinline__ void row_transform(uint32_t (&va)[1 << LV], uint32_t 
             pass_load<KP, WL, LV>(vb, sb, tid, T, logd);
         }
         pass_forward<KP, WL, LV>(va, vb, tid, T, s0, logd, stf, pc.p, pc.two_p);
-        if (q + 1 < NP || REM) {
-            pass_store<KP, WL, LV>(va, sa, tid, T, logd);
-            pass_store<KP, WL, LV>(vb, sb, tid, T, logd);
-            const bool next_local =
-                q + 1 < NP ? pass_warp_local<KP, WL, LV>(logd - KP) : pass_warp_local<KR, WL, LV>(0);
-            exchange_sync(pass_warp_local<KP, WL, LV>(logd) && next_local);
+        pass_store<KP, WL, LV>(va, sa, tid, T, logd);
+        pass_store<KP, WL, LV>(vb, sb, tid, T, logd);
+        const bool next_local =
+            q + 1 < NP ? pass_warp_local<KP, WL, LV>(logd - KP) : (MID ? mid_local : close_local);
+        exchange_sync(pass_warp_local<KP, WL, LV>(logd) && next_local);
+    }
+    if constexpr (MID > 0) {
+        if (NP > 0) {
+            pass_load<KM, WL, LV>(va, sa, tid, T, kDeferred);
+            pass_load<KM, WL, LV>(vb, sb, tid, T, kDeferred);
+        }
+        pass_forward<KM, WL, LV>(va, vb, tid, T, KP * NP, kDeferred, stf, pc.p, pc.two_p);
+        pass_store<KM, WL, LV>(va, sa, tid, T, kDeferred);
+        pass_store<KM, WL, LV>(vb, sb, tid, T, kDeferred);
+        exchange_sync(mid_local && close_local);
+    }
+    constexpr int sc = LOGC - KC;  // the closing pass's first stage
+    if constexpr (NP > 0 || MID > 0) {
+        pass_load<KC, WL, LV>(va, sa, tid, T, 0);
+        pass_load<KC, WL, LV>(vb, sb, tid, T, 0);
+    }
+    if constexpr (CL > 0) pass_forward<KC, WL, LV, CL>(va, vb, tid, T, sc, 0, stf, pc.p, pc.two_p);
+    // --- products: quad b of the row is modulo X^4 - zeta, zeta = +w (b even) or -w (b odd), w the
+    // twiddle of the butterfly that split it from its sibling (times 2^-32, which the CRT scale removes)
+#pragma unroll
+    for (int m = 0; m < ((1 << LV) >> KC); ++m) {
+        const int b0 = pass_gid<KC, WL, LV>(tid, T, m) << CL;
+#pragma unroll
+        for (int t = 0; t < (1 << CL); ++t) {
+            uint2 zeta = stf[(1 << (LOGC - 3)) + ((b0 + t) >> 1)];
+            if ((b0 + t) & 1) zeta = shoup_negate(zeta, pc.p);
+            const int e = (m << KC) + 4 * t;
+            quad_product(va[e], va[e + 1], va[e + 2], va[e + 3], vb[e], vb[e + 1], vb[e + 2], vb[e + 3], zeta, pc.p,
+                         pc.two_p, pc.pinv);
         }
     }
-    if constexpr (REM > 0) {
-        const int s0 = KP * NP, logd = 0;
-        pass_load<REM, WL, LV>(va, sa, tid, T, logd);
-        pass_load<REM, WL, LV>(vb, sb, tid, T, logd);
-        pass_forward<REM, WL, LV>(va, vb, tid, T, s0, logd, stf, pc.p, pc.two_p);
+    // --- inverse ---
+    if constexpr (CL > 0) {
+        if constexpr (NP == 0 && MID == 0) after_last_load();
+        pass_inverse<KC, WL, LV, CL>(va, tid, T, sc, 0, sti, pc.p, pc.two_p);
     }
-    // pointwise product in Montgomery form (a factor 2^-32 the CRT scale removes), in [0, 2p)
-#pragma unroll
-    for (int l = 0; l < (1 << LV); ++l)
-        va[l] = mont_mul(csub(va[l], pc.two_p), csub(vb[l], pc.two_p), pc.p, pc.pinv);
-    if constexpr (REM > 0) {
-        const int s0 = KP * NP, logd = 0;
-        pass_inverse<REM, WL, LV>(va, tid, T, s0, logd, sti, pc.p, pc.two_p);
-        pass_store<REM, WL, LV>(va, sa, tid, T, logd);
-        exchange_sync(pass_warp_local<REM, WL, LV>(0) && pass_warp_local<KP, WL, LV>(LOGC - KP * NP));
+    if constexpr (NP > 0 || MID > 0) {
+        pass_store<KC, WL, LV>(va, sa, tid, T, 0);
+        exchange_sync(close_local && (MID ? mid_local : pass_warp_local<KP, WL, LV>(LOGC - KP * NP)));
+    }
+    if constexpr (MID > 0) {
+        pass_load<KM, WL, LV>(va, sa, tid, T, kDeferred);
+        if constexpr (NP == 0) after_last_load();
+        pass_inverse<KM, WL, LV>(va, tid, T, KP * NP, kDeferred, sti, pc.p, pc.two_p);
+        if constexpr (NP > 0) {
+            pass_store<KM, WL, LV>(va, sa, tid, T, kDeferred);
+            exchange_sync(mid_local && pass_warp_local<KP, WL, LV>(LOGC - KP * NP));
+        }
     }
 #pragma unroll
     for (int q = NP - 1; q >= 0; --q) {
         const int s0 = KP * q, logd = LOGC - s0 - KP;
-        if (q + 1 < NP || REM) pass_load<KP, WL, LV>(va, sa, tid, T, logd);
+        pass_load<KP, WL, LV>(va, sa, tid, T, logd);
         if (q == 0) after_last_load();
         pass_inverse<KP, WL, LV>(va, tid, T, s0, logd, sti, pc.p, pc.two_p);
         if (q > 0) {
@@ -285,14 +336,13 @@ __device__ __forceinline__ void row_transform(uint32_t (&va)[1 << LV], uint32_t 
 constexpr int k2_threads(int logc) { return logc >= 12 ? 512 : (logc >= 11 ? 256 : 128); }
 constexpr int k2_min_blocks(int logc) { return logc >= 12 ? 1 : (logc >= 11 ? 3 : 7); }
 
-// Rows of C = 2^LOGC >= 8, passes of KP stages (radix 2^KP, KP = 2 or 3; the
-// last forward pass takes the remaining LOGC % KP stages).  grid
-// (R / rows_per_cta, P, count), block rows_per_cta * C/8.  Dynamic shared
-// memory per row: C uint2 forward and C uint2 inverse twiddles, then 2C words
-// of data.  The product overwrites the a plane in place.
+// Rows of C = 2^LOGC >= 8, passes of KP stages (radix 2^KP, KP = 2 or 3; see
+// RowPlan).  grid (R / rows_per_cta, P, count), block rows_per_cta * C/8.
+// Dynamic shared memory per row: C/4 uint2 forward and C/4 uint2 inverse
+// twiddles, then 2C words of data.  The product overwrites the a plane in place.
 // One row r of prime i of the residue planes at `res` ([2][P][n]); the calling
 // CTA gives each row T = C/8 threads (sub = row slot in the CTA, tid = thread in
-// the row) and 24*C bytes of dynamic shared memory per row slot.
+// the row) and 12*C bytes of dynamic shared memory per row slot.
 template <int LOGC, int KP>
 __device__ __forceinline__ void k2_row_body(uint32_t* __restrict__ res, const PrimeConst& pc,
                                             const uint2* __restrict__ tw_fwd, const uint2* __restrict__ tw_inv,
@@ -303,28 +353,30 @@ __device__ __forceinline__ void k2_row_body(uint32_t* __restrict__ res, const Pr
     static_assert(KP == 2 || KP == 3, "pass radix");
     extern __shared__ __align__(16) uint2 smem2[];
     const int R = 1 << logR;
-    uint2* stf = smem2 + sub * 2 * C;
-    uint2* sti = stf + C;
-    uint32_t* sa = reinterpret_cast<uint32_t*>(smem2 + rows_per_cta * 2 * C) + sub * 2 * C;
+    using Plan = RowPlan<LOGC, KP, 3>;
+    constexpr int TW = C / 4;  // twiddles of the row's LOGC - 2 stages
+    uint2* stf = smem2 + sub * 2 * TW;
+    uint2* sti = stf + TW;
+    uint32_t* sa = reinterpret_cast<uint32_t*>(smem2 + rows_per_cta * 2 * TW) + sub * 2 * C;
     uint32_t* sb = sa + C;
     uint32_t* ga = res + size_t(i) * n + size_t(r) * C;
     const uint32_t* gb = res + size_t(P + i) * n + size_t(r) * C;
-    constexpr int logd0 = LOGC - KP;  // first pass: s0 = 0
+    constexpr int K0 = Plan::K0, logd0 = Plan::LOGD0;
 
     uint32_t va[8], vb[8];
 #pragma unroll
-    for (int m = 0; m < (8 >> KP); ++m)
+    for (int m = 0; m < (8 >> K0); ++m)
 #pragma unroll
-        for (int l = 0; l < (1 << KP); ++l) {
-            const int idx = pass_index<KP>(tid, T, m, l, logd0);
-            va[(m << KP) + l] = ga[idx];
-            vb[(m << KP) + l] = gb[idx];
+        for (int l = 0; l < (1 << K0); ++l) {
+            const int idx = pass_index<K0>(tid, T, m, l, logd0);
+            va[(m << K0) + l] = ga[idx];
+            vb[(m << K0) + l] = gb[idx];
         }
     // this row's twiddles: local entry j = 2^s + i' holds Psi_rev[(R + r) 2^s + i']
     {
         const uint2* gf = tw_fwd + size_t(i) * kNMax;
         const uint2* gi = tw_inv + size_t(i) * kNMax;
-        for (int j = tid; j < C; j += T) {
+        for (int j = tid; j < TW; j += T) {
             if (j == 0) continue;
             const int s = 31 - __clz(j);
             const int gidx = ((R + r) << s) + (j - (1 << s));
@@ -335,9 +387,9 @@ __device__ __forceinline__ void k2_row_body(uint32_t* __restrict__ res, const Pr
     __syncthreads();
     row_transform<LOGC, KP>(va, vb, sa, sb, stf, sti, tid, pc);
 #pragma unroll
-    for (int m = 0; m < (8 >> KP); ++m)
+    for (int m = 0; m < (8 >> K0); ++m)
 #pragma unroll
-        for (int l = 0; l < (1 << KP); ++l) ga[pass_index<KP>(tid, T, m, l, logd0)] = va[(m << KP) + l];
+        for (int l = 0; l < (1 << K0); ++l) ga[pass_index<K0>(tid, T, m, l, logd0)] = va[(m << K0) + l];
 }
 
 template <int LOGC, int KP>
@@ -352,11 +404,12 @@ __global__ void __launch_bounds__(k2_threads(LOGC), k2_min_blocks(LOGC))
                           blockIdx.x * rows_per_cta + sub, sub, tid, rows_per_cta);
 }
 
-// Rows of C <= 4 (N <= 128): one thread per row, everything in registers.
+// Rows of C <= 4 (N <= 128): one thread per row, one product of polynomials of C values
+// (every row stage is deferred).  Row r ended the column stages as the residue modulo
+// X^C - zeta, zeta = +-Psi_rev[(R + r) / 2] (the butterfly that split it from row r ^ 1).
 // grid ((R+31)/32, P, count).
 static __global__ void k2_rows_small(uint32_t* __restrict__ res, const PrimeConst* __restrict__ pcs,
-                              const uint2* __restrict__ tw_fwd, const uint2* __restrict__ tw_inv, int n, int logR,
-                              int logC, int P, size_t ws_bstride) {
+                              const uint2* __restrict__ tw_fwd, int n, int logR, int logC, int P, size_t ws_bstride) {
     const int R = 1 << logR, C = 1 << logC;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
@@ -365,45 +418,15 @@ static __global__ void k2_rows_small(uint32_t* __restrict__ res, const PrimeCons
     res += blockIdx.z * ws_bstride;
     uint32_t* ga = res + size_t(i) * n + size_t(r) * C;
     const uint32_t* gb = res + size_t(P + i) * n + size_t(r) * C;
-    const uint2* twf = tw_fwd + size_t(i) * kNMax;
-    const uint2* twi = tw_inv + size_t(i) * kNMax;
-    uint32_t va[4], vb[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        va[j] = j < C ? ga[j] : 0;
-        vb[j] = j < C ? gb[j] : 0;
+    uint2 zeta = tw_fwd[size_t(i) * kNMax + ((R + r) >> 1)];
+    if (r & 1) zeta = shoup_negate(zeta, pc.p);
+    if (C == 4) {
+        quad_product(ga[0], ga[1], ga[2], ga[3], gb[0], gb[1], gb[2], gb[3], zeta, pc.p, pc.two_p, pc.pinv);
+    } else if (C == 2) {
+        pair_product(ga[0], ga[1], gb[0], gb[1], zeta, pc.p, pc.two_p, pc.pinv);
+    } else {
+        ga[0] = mont_mul(csub(ga[0], pc.two_p), csub(gb[0], pc.two_p), pc.p, pc.pinv);
     }
-    for (int s = 0; s < logC; ++s) {
-        const int t = C >> (s + 1);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j < C && !(j & t)) {
-                const uint2 w = twf[((R + r) << s) + (j >> (logC - s))];
-                // register indices must be compile-time; select the partner explicitly
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (k == j + t) {
-                        ct_bfly(va[j], va[k], w, pc.p, pc.two_p);
-                        ct_bfly(vb[j], vb[k], w, pc.p, pc.two_p);
-                    }
-            }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) va[j] = mont_mul(csub(va[j], pc.two_p), csub(vb[j], pc.two_p), pc.p, pc.pinv);
-    for (int s = logC - 1; s >= 0; --s) {
-        const int t = C >> (s + 1);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j < C && !(j & t)) {
-                const uint2 w = twi[((R + r) << s) + (j >> (logC - s))];
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (k == j + t) gs_bfly(va[j], va[k], w, pc.p, pc.two_p);
-            }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (j < C) ga[j] = va[j];
 }
 
 // ---------------------------------------------------------------------------

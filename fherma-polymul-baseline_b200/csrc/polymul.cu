@@ -327,7 +327,8 @@ void PlanCore::init(uint32_t n_, const uint64_t* q64, uint32_t q_limbs, uint32_t
     P = basis_size(basis->primes, n, qbits);
 
     // CRT constants: (P_total / p_i) mod q, (-P_total) mod q,
-    // scale = 2^32 n^-1 (P/p_i)^-1 mod p_i (2^32 undoes the Montgomery product of K2)
+    // scale = 2^32 (n / 4)^-1 (P/p_i)^-1 mod p_i (2^32 undoes the Montgomery product of K2, n / 4 the
+    // doublings of the inverse stages: the rows defer two, in rows of 2 values one, of 1 none)
     Words total{1};
     for (unsigned i = 0; i < P; ++i) total = multiply_small(total, basis->primes[i]);
     std::vector<uint32_t> mq(size_t(P) * W, 0), consts(2 * size_t(W), 0);
@@ -339,7 +340,7 @@ void PlanCore::init(uint32_t n_, const uint64_t* q64, uint32_t q_limbs, uint32_t
         const Words mmod = padded(mod(m, q), W);
         std::copy(mmod.begin(), mmod.end(), mq.begin() + size_t(i) * W);
         const uint32_t minv = powmod(mod_small(m, p), p - 2, p);
-        const uint32_t ninv = powmod(n % p, p - 2, p);
+        const uint32_t ninv = powmod((n >> deferred_stages(int(logC))) % p, p - 2, p);
         const uint32_t r32 = uint32_t((uint64_t(1) << 32) % p);
         const uint32_t s = mulmod(mulmod(minv, ninv, p), r32, p);
         scale[i] = make_uint2(s, shoup_of(s, p));
@@ -480,7 +481,7 @@ void launch_k2_fixed(const PlanCore& s, uint32_t* work, const Batch& bt, cudaStr
         int rows = T >= 128 ? 1 : 128 / T;
         const int R = 1 << s.logR;
         if (rows > R) rows = R;
-        const size_t smem = size_t(rows) * 24 * C;  // 2C uint2 twiddles + 2C words of data per row
+        const size_t smem = size_t(rows) * 12 * C;  // C/2 uint2 twiddles + 2C words of data per row
         if (smem > 48 * 1024)
             cuda_check(cudaFuncSetAttribute(k2_rows<LOGC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
                        "raise K2 shared memory");
@@ -515,8 +516,8 @@ void launch_k2(const PlanCore& s, uint32_t* work, const Batch& bt, cudaStream_t 
         default: {
             const int R = 1 << s.logR;
             dim3 grid((R + 31) / 32, s.P, bt.count), block(R < 32 ? R : 32);
-            k2_rows_small<<<grid, block, 0, st>>>(work, s.plane_pc(), s.plane_fwd(), s.plane_inv(),
-                                                 int(s.n), int(s.logR), int(s.logC), int(s.P), bt.ws_bstride);
+            k2_rows_small<<<grid, block, 0, st>>>(work, s.plane_pc(), s.plane_fwd(), int(s.n), int(s.logR),
+                                                 int(s.logC), int(s.P), bt.ws_bstride);
         }
     }
 }

@@ -203,11 +203,11 @@ void quartic_init(PlanCore& s) {
                 put(112u + unsigned(t), (rho_m[m] + p - wrong) % p);
             }
         }
-        // CRT: s_i = 2^32 n^-1 (P/p_i)^-1, component scales s_i r^-m / 4
+        // CRT: s_i = 2^32 (n / 4)^-1 (P/p_i)^-1 (the row kernels defer two stages), component scales s_i r^-m / 4
         Words Mi = P;
         divide_small(Mi, p);
         const uint32_t minv = powmod(mod_small(Mi, p), p - 2, p);
-        const uint32_t ninv = powmod(s.n % p, p - 2, p);
+        const uint32_t ninv = powmod((s.n >> deferred_stages(int(s.logC))) % p, p - 2, p);
         const uint32_t si = mulmod(mulmod(minv, ninv, p), uint32_t((uint64_t(1) << 32) % p), p);
         const uint32_t rinv = powmod(r, p - 2, p), inv4 = powmod(4, p - 2, p);
         const uint32_t iinv = powmod(iota, p - 2, p);

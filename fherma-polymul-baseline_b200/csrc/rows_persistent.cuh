@@ -7,7 +7,7 @@
 // of one plan (pair = i * R + r, item = pair * count + z); a batch of products
 // of one row size but different q reads them from a table.  Each CTA owns a contiguous range of
 // items and, for each of them:
-//   - stages the pair's 2C forward/inverse row twiddles with bulk copies, only
+//   - stages the pair's C/4 + C/4 forward/inverse row twiddles with bulk copies, only
 //     when the pair changes (once per pair instead of once per product);
 //   - has the item's two rows (a and b, 4C bytes each) in shared memory already:
 //     they were requested by bulk copy while the previous item was finishing;
@@ -16,16 +16,15 @@
 //     every thread holds the values of the last pass, the buffer is free and
 //     the next item's rows are requested into it, landing while this item's
 //     last stages run and its product row is stored.
-// One data buffer instead of two keeps a CTA at 48 KB (C = 2048), so four CTAs
-// share an SM; at C = 4096, 96 KB and two.  One row per CTA, C >= 1024, with
+// A CTA takes 24 KB (C = 2048); four share an SM (registers), two at C = 4096.  One row per CTA, C >= 1024, with
 // T = C/16 threads of 16 values (radix-16 passes, the default: two exchanges
 // per direction instead of three, up to 128 registers a thread) or T = C/8
 // threads of 8 values (radix 4 or 8, at most 64 registers).  Bulk copies need
 // 16-byte aligned rows: the host launches this kernel only on 16-byte aligned
 // workspaces.
 //
-// Dynamic shared memory: C uint2 forward and C uint2 inverse twiddles, one data
-// buffer of 2C words, two mbarriers (data, twiddles): 24C + 16 B.
+// Dynamic shared memory: C/4 uint2 forward and C/4 uint2 inverse twiddles, one data
+// buffer of 2C words, two mbarriers (data, twiddles): 12C + 16 B.
 #pragma once
 
 #include <cstdint>
@@ -58,7 +57,7 @@ constexpr int k2p_min_blocks(int logc) { return logc >= 12 ? 2 : (logc >= 11 ? 4
 // values a thread: 16 for radix-16 passes (KP = 4), else 8
 constexpr int k2p_lv(int kp) { return kp == 4 ? 4 : 3; }
 constexpr int k2p_threads(int logc, int kp) { return (1 << logc) >> k2p_lv(kp); }
-constexpr size_t k2p_smem_bytes(int logc) { return (size_t(24) << logc) + 2 * sizeof(uint64_t); }
+constexpr size_t k2p_smem_bytes(int logc) { return (size_t(12) << logc) + 2 * sizeof(uint64_t); }
 
 template <int LOGC, int KP, class Work>
 __global__ void __launch_bounds__(k2p_threads(LOGC, KP), k2p_min_blocks(LOGC))
@@ -66,12 +65,14 @@ __global__ void __launch_bounds__(k2p_threads(LOGC, KP), k2p_min_blocks(LOGC))
              const uint2* __restrict__ tw_inv, int logR, uint32_t* __restrict__ err) {
     constexpr int LV = k2p_lv(KP), V = 1 << LV;
     constexpr int C = 1 << LOGC, T = C >> LV;
-    constexpr int logd0 = LOGC - KP;  // first pass: s0 = 0
+    using Plan = RowPlan<LOGC, KP, LV>;
+    constexpr int K0 = Plan::K0, logd0 = Plan::LOGD0;
+    constexpr int TW = C / 4;  // twiddles of the row's LOGC - 2 stages
     static_assert(LOGC >= 10, "one row per CTA needs C >= 1024");
     extern __shared__ __align__(16) uint2 smem2[];
     uint2* stf = smem2;
-    uint2* sti = smem2 + C;
-    uint32_t* sd = reinterpret_cast<uint32_t*>(smem2 + 2 * C);  // [2C] words
+    uint2* sti = smem2 + TW;
+    uint32_t* sd = reinterpret_cast<uint32_t*>(smem2 + 2 * TW);  // [2C] words
     uint64_t* bars = reinterpret_cast<uint64_t*>(sd + 2 * C);   // data, twiddles
 
     const int tid = threadIdx.x;
@@ -120,8 +121,8 @@ __global__ void __launch_bounds__(k2p_threads(LOGC, KP), k2p_min_blocks(LOGC))
                 const uint2* gi = tw_inv + size_t(i) * kNMax;
                 // local entry j = 2^s + i' holds Psi_rev[(R + r) 2^s + i']; stage s > 0 is one
                 // contiguous, 16-byte aligned run of 2^s entries, stage 0 a single entry
-                tc::mbar_expect_tx(&bars[1], 16u * uint32_t(C - 2));
-                for (int s = 1; s < LOGC; ++s) {
+                tc::mbar_expect_tx(&bars[1], 16u * uint32_t(TW - 2));
+                for (int s = 1; s < LOGC - kDeferred; ++s) {
                     tc::bulk_load(stf + (1 << s), gf + (size_t(R + r) << s), 8u << s, &bars[1]);
                     tc::bulk_load(sti + (1 << s), gi + (size_t(R + r) << s), 8u << s, &bars[1]);
                 }
@@ -140,12 +141,12 @@ __global__ void __launch_bounds__(k2p_threads(LOGC, KP), k2p_min_blocks(LOGC))
         uint32_t* sb = sa + C;
         uint32_t va[V], vb[V];
 #pragma unroll
-        for (int m = 0; m < (V >> KP); ++m)
+        for (int m = 0; m < (V >> K0); ++m)
 #pragma unroll
-            for (int l = 0; l < (1 << KP); ++l) {
-                const int idx = pass_index<KP, false, LV>(tid, T, m, l, logd0);
-                va[(m << KP) + l] = sa[idx];
-                vb[(m << KP) + l] = sb[idx];
+            for (int l = 0; l < (1 << K0); ++l) {
+                const int idx = pass_index<K0, false, LV>(tid, T, m, l, logd0);
+                va[(m << K0) + l] = sa[idx];
+                vb[(m << K0) + l] = sb[idx];
             }
         // the rows arrived unswizzled and the exchanges store swizzled: every thread
         // has its values before any exchange store lands in this buffer (and a wait
@@ -163,9 +164,9 @@ __global__ void __launch_bounds__(k2p_threads(LOGC, KP), k2p_min_blocks(LOGC))
         row_transform<LOGC, KP, decltype(hook), LV>(va, vb, sa, sb, stf, sti, tid, pc, hook);
         uint32_t* ga = it.a;
 #pragma unroll
-        for (int m = 0; m < (V >> KP); ++m)
+        for (int m = 0; m < (V >> K0); ++m)
 #pragma unroll
-            for (int l = 0; l < (1 << KP); ++l) ga[pass_index<KP, false, LV>(tid, T, m, l, logd0)] = va[(m << KP) + l];
+            for (int l = 0; l < (1 << K0); ++l) ga[pass_index<K0, false, LV>(tid, T, m, l, logd0)] = va[(m << K0) + l];
     }
     // after a wait gave up (and the loop stopped): copies already requested land
     // before the CTA's shared memory goes away; no new copies were requested
