@@ -109,7 +109,7 @@ Tuning autotune(PlanCore& s, uint32_t reps, double* us_per_product) {
             best = t;
         }
     };
-    if (s.logC >= 10) {
+    if (s.logC >= 4) {
         Tuning t = best;
         t.row_persistent = !best.row_persistent;
         consider(t);
@@ -117,6 +117,7 @@ Tuning autotune(PlanCore& s, uint32_t reps, double* us_per_product) {
     if (s.logC >= 4) {
         for (int radix : {2, 3, 4}) {
             if (radix == 4 && !(s.logC >= 10 && best.row_persistent)) continue;  // radix-16: persistent kernel only
+            if (s.logC < 10 && best.row_persistent) continue;  // the warp kernel's passes are fixed
             Tuning t = best;
             t.row_radix_log = radix;
             if (radix != best.row_radix_log) consider(t);

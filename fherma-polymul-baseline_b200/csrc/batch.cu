@@ -10,7 +10,7 @@
 //                     launch per class: the persistent k2p_rows for rows of
 //                     1024 values or more (items prime/row first, so a CTA
 //                     stages a row's twiddles once for every product that
-//                     has it), k2_rows_items for shorter rows;
+//                     has it), k2w_rows for shorter rows;
 //   CRT items         (product, column group) per width class -- one persistent
 //                     launch of k3t_crt per class.
 // These launches are captured into a CUDA graph (the classes of a phase on
@@ -28,26 +28,12 @@
 #include "../../include/polymul.h"
 #include "pm_internal.h"
 #include "rows_persistent.cuh"
+#include "rows_warp.cuh"
 #include "tensor_kernels.cuh"
 
 namespace pm {
 
-// rows of a class, (product, prime, first row) items; one CTA per item
-template <int LOGC, int KP>
-__global__ void __launch_bounds__(k2_threads(LOGC), k2_min_blocks(LOGC))
-    k2_rows_items(const uint4* __restrict__ items, const BatchProduct* __restrict__ prod, uint32_t* __restrict__ work,
-                  const PrimeConst* __restrict__ pcs, const uint2* __restrict__ tw_fwd,
-                  const uint2* __restrict__ tw_inv, int logR) {
-    constexpr int T = (1 << LOGC) / 8;
-    const uint4 it = items[blockIdx.x];
-    const BatchProduct& d = prod[it.x];
-    const int sub = threadIdx.x / T, tid = threadIdx.x % T;
-    const int rows_per_cta = blockDim.x / T;
-    k2_row_body<LOGC, KP>(work + d.ws_off, pcs[it.y], tw_fwd, tw_inv, d.n, logR, d.P, int(it.y), int(it.z) + sub,
-                          sub, tid, rows_per_cta);
-}
-
-// rows of one size class from a table of (product, prime, row) items
+// rows of one size class from a table of (product, prime, first row) items
 struct TableRowWork {
     const uint4* items;
     int nitems;
@@ -96,52 +82,49 @@ CUtensorMap encode(CUtensorMapDataType type, const void* base, const cuuint64_t 
 }
 
 template <int LOGC, int KP>
-void launch_rows_class(const uint4* items, int count, int rows_per_item, const BatchProduct* prod, uint32_t* work,
-                       const DeviceBasis& B, uint32_t* err, cudaStream_t st) {
-    constexpr int C = 1 << LOGC, T = C / 8;
+void launch_rows_class(const uint4* items, int count, const BatchProduct* prod, uint32_t* work, const DeviceBasis& B,
+                       uint32_t* err, cudaStream_t st) {
+    const TableRowWork w{items, count, prod, work};
     if constexpr (LOGC >= 10) {
         const size_t smem = k2p_smem_bytes(LOGC);
         cuda_check(cudaFuncSetAttribute(k2p_rows<LOGC, KP, TableRowWork>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(smem)),
                    "batch row shared memory");
-        const TableRowWork w{items, count, prod, work};
         const int ctas = std::min(count, sm_count_dev() * k2p_min_blocks(LOGC));
         k2p_rows<LOGC, KP, TableRowWork><<<ctas, k2p_threads(LOGC, KP), smem, st>>>(w, B.d_pc, B.d_tw_fwd,
                                                                                     B.d_tw_inv, 4, err);
     } else {
-        const size_t smem = size_t(rows_per_item) * 12 * C;
-        if (smem > 48 * 1024)
-            cuda_check(cudaFuncSetAttribute(k2_rows_items<LOGC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            int(smem)),
-                       "batch row shared memory");
-        k2_rows_items<LOGC, KP><<<count, rows_per_item * T, smem, st>>>(items, prod, work, B.d_pc, B.d_tw_fwd,
-                                                                        B.d_tw_inv, 4);
+        k2w_rows<LOGC, TableRowWork><<<k2w_grid(count, sm_count_dev()), 32 * kWarpRowWarps, k2w_smem_bytes<LOGC>(),
+                                       st>>>(w, B.d_pc, B.d_tw_fwd, B.d_tw_inv, 4);
     }
 }
 
+// radix_log: the register-pass radix of the persistent kernel's rows (C >= 1024)
 template <int LOGC>
-void launch_rows_radix(int radix_log, const uint4* items, int count, int rows, const BatchProduct* prod,
-                       uint32_t* work, const DeviceBasis& B, uint32_t* err, cudaStream_t st) {
-    if (radix_log == 2)
-        launch_rows_class<LOGC, 2>(items, count, rows, prod, work, B, err, st);
-    else if (LOGC >= 10 && radix_log == 4)  // radix-16 passes: the persistent kernel only
-        launch_rows_class<LOGC, LOGC >= 10 ? 4 : 3>(items, count, rows, prod, work, B, err, st);
+void launch_rows_radix(int radix_log, const uint4* items, int count, const BatchProduct* prod, uint32_t* work,
+                       const DeviceBasis& B, uint32_t* err, cudaStream_t st) {
+    if constexpr (LOGC < 10)
+        launch_rows_class<LOGC, 4>(items, count, prod, work, B, err, st);
+    else if (radix_log == 2)
+        launch_rows_class<LOGC, 2>(items, count, prod, work, B, err, st);
+    else if (radix_log == 3)
+        launch_rows_class<LOGC, 3>(items, count, prod, work, B, err, st);
     else
-        launch_rows_class<LOGC, 3>(items, count, rows, prod, work, B, err, st);
+        launch_rows_class<LOGC, 4>(items, count, prod, work, B, err, st);
 }
 
-void launch_rows_any(int logC, int radix_log, const uint4* items, int count, int rows, const BatchProduct* prod,
+void launch_rows_any(int logC, int radix_log, const uint4* items, int count, const BatchProduct* prod,
                      uint32_t* work, const DeviceBasis& B, uint32_t* err, cudaStream_t st) {
     switch (logC) {
-        case 4: return launch_rows_radix<4>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 5: return launch_rows_radix<5>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 6: return launch_rows_radix<6>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 7: return launch_rows_radix<7>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 8: return launch_rows_radix<8>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 9: return launch_rows_radix<9>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 10: return launch_rows_radix<10>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 11: return launch_rows_radix<11>(radix_log, items, count, rows, prod, work, B, err, st);
-        case 12: return launch_rows_radix<12>(radix_log, items, count, rows, prod, work, B, err, st);
+        case 4: return launch_rows_radix<4>(radix_log, items, count, prod, work, B, err, st);
+        case 5: return launch_rows_radix<5>(radix_log, items, count, prod, work, B, err, st);
+        case 6: return launch_rows_radix<6>(radix_log, items, count, prod, work, B, err, st);
+        case 7: return launch_rows_radix<7>(radix_log, items, count, prod, work, B, err, st);
+        case 8: return launch_rows_radix<8>(radix_log, items, count, prod, work, B, err, st);
+        case 9: return launch_rows_radix<9>(radix_log, items, count, prod, work, B, err, st);
+        case 10: return launch_rows_radix<10>(radix_log, items, count, prod, work, B, err, st);
+        case 11: return launch_rows_radix<11>(radix_log, items, count, prod, work, B, err, st);
+        case 12: return launch_rows_radix<12>(radix_log, items, count, prod, work, B, err, st);
         default: throw Failure(PM_ERR_UNSUPPORTED, "row size outside the batch kernels");
     }
 }
@@ -188,7 +171,7 @@ struct BatchCore {
     uint32_t* d_err = nullptr;
     int conv_items = 0;
     struct RowClass {
-        int logC, radix_log, rows, count;
+        int logC, radix_log, count;
         size_t offset;  // into d_row_items
     };
     struct CrtClass {
@@ -242,7 +225,7 @@ struct BatchCore {
         for (size_t k = 0; k < row_classes.size(); ++k) {
             const RowClass& rc = row_classes[k];
             cudaStream_t s = fork(k);
-            launch_rows_any(rc.logC, rc.radix_log, d_row_items + rc.offset, rc.count, rc.rows, d_prod, d_work, B, d_err,
+            launch_rows_any(rc.logC, rc.radix_log, d_row_items + rc.offset, rc.count, d_prod, d_work, B, d_err,
                             s);
             used.push_back(s);
         }
@@ -333,28 +316,24 @@ struct BatchCore {
             }
         conv_items = int(conv.size());
         std::map<int, std::vector<uint4>> rows_by_c;
-        std::map<int, int> rows_per_item;
         for (uint32_t z = 0; z < cnt; ++z) {
             const PlanCore& p = *plans[z];
-            const int T = (1 << p.logC) / 8, R = 1 << p.logR;
-            int rows = T >= 128 ? 1 : 128 / T;
-            if (rows > R) rows = R;
-            rows_per_item[int(p.logC)] = rows;
+            const int R = 1 << p.logR, rows = p.logC >= 10 ? 1 : warp_rows(int(p.logC), int(p.logR));
             for (uint32_t i = 0; i < p.P; ++i)
                 for (int r = 0; r < R; r += rows) rows_by_c[int(p.logC)].push_back(make_uint4(z, i, uint32_t(r), 0));
         }
         std::vector<uint4> row_items;
         for (auto& [logC, items] : rows_by_c) {
-            if (logC >= 10)  // the persistent row kernel: consecutive items share a (prime, row) pair
-                std::stable_sort(items.begin(), items.end(), [](const uint4& x, const uint4& y) {
-                    return x.y != y.y ? x.y < y.y : x.z < y.z;
-                });
+            // consecutive items share their (prime, rows): the row kernels keep their twiddles
+            std::stable_sort(items.begin(), items.end(), [](const uint4& x, const uint4& y) {
+                return x.y != y.y ? x.y < y.y : x.z < y.z;
+            });
             // the radix the autotuner picked for plans of this row size; by default radix 16
-            // for the persistent kernel's rows (C >= 1024), radix 8 below
-            int radix_log = logC >= 10 ? 4 : 3;
+            // (rows of C >= 1024; shorter rows' passes are fixed)
+            int radix_log = 4;
             for (auto& p : plans)
                 if (int(p->logC) == logC && p->tune.tuned) radix_log = p->tune.row_radix_log;
-            row_classes.push_back(RowClass{logC, radix_log, rows_per_item[logC], int(items.size()), row_items.size()});
+            row_classes.push_back(RowClass{logC, radix_log, int(items.size()), row_items.size()});
             row_items.insert(row_items.end(), items.begin(), items.end());
         }
         std::map<int, std::vector<uint2>> crt_by_w;
@@ -447,7 +426,7 @@ struct BatchCore {
         for (auto& rc : row_classes)
             for (int k : {2, 3, 4}) {
                 const int cur = rc.radix_log;
-                if (k == cur || (k == 4 && rc.logC < 10)) continue;  // radix 16: persistent kernel rows only
+                if (k == cur || rc.logC < 10) continue;  // the warp kernel's passes are fixed
                 attempt([&] { rc.radix_log = k; }, [&] { rc.radix_log = cur; });
             }
         for (int k : {2, 3, 4}) {

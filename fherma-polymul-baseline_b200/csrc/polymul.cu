@@ -17,6 +17,7 @@
 #include "pm_device.cuh"
 #include "pm_internal.h"
 #include "rows_persistent.cuh"
+#include "rows_warp.cuh"
 
 namespace pm {
 
@@ -459,6 +460,17 @@ void launch_k3(const PlanCore& s, const uint32_t* work, uint32_t* c, const Batch
 template <int LOGC, int KP>
 void launch_k2_fixed(const PlanCore& s, uint32_t* work, const Batch& bt, cudaStream_t st) {
     constexpr int C = 1 << LOGC, T = C / 8;
+    if constexpr (LOGC >= 4 && LOGC <= 9) {
+        // rows of 16 .. 512 values, a warp at a time (16-byte runs of aligned rows)
+        if (s.tune.row_persistent && (reinterpret_cast<uintptr_t>(work) & 15) == 0 && (bt.ws_bstride & 3) == 0) {
+            const size_t smem = k2w_smem_bytes<LOGC>();
+            const PlanWarpRowWork w{work, bt.ws_bstride, int(s.n), int(s.logR), int(s.logC), int(s.P), int(bt.count)};
+            const int64_t items = int64_t(s.P) * ((1 << s.logR) / warp_rows(LOGC, int(s.logR))) * bt.count;
+            k2w_rows<LOGC, PlanWarpRowWork><<<k2w_grid(items, s.sms), 32 * kWarpRowWarps, smem, st>>>(
+                w, s.plane_pc(), s.plane_fwd(), s.plane_inv(), int(s.logR));
+            return;
+        }
+    }
     if constexpr (LOGC >= 10) {
         // bulk copies need 16-byte aligned rows (n, C and the product stride are multiples of 4 words)
         if (s.tune.row_persistent && (reinterpret_cast<uintptr_t>(work) & 15) == 0 && (bt.ws_bstride & 3) == 0) {

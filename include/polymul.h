@@ -99,8 +99,9 @@ typedef struct {
     uint32_t crt_ctas_per_sm;   /* persistent CTAs of the tensor CRT per SM, 1..4 */
     uint32_t group;             /* products per launch group in batched calls (0: up to ~2 GB of residues and
                                    128 products; at most 256) */
-    uint32_t row_persistent;    /* 1: rows of >= 1024 values by the persistent kernel that stages a row's
-                                   twiddles once per group and prefetches rows; 0: one CTA per row */
+    uint32_t row_persistent;    /* 1: the kernels that stage a row's twiddles once per group of products (rows
+                                   of >= 1024 values: one CTA each, prefetched; of 16 .. 512: a warp per 512
+                                   values, row_radix unused); 0: CTAs per row, twiddles read per product */
     uint32_t conv_whole_basis;  /* tensor conversion: 1 (the default) takes each coefficient tile through all
                                    primes at once (weights of the whole basis resident, 2 CTAs per SM;
                                    conv_ctas_per_sm unused); 0 runs it once per group of 16 primes */
