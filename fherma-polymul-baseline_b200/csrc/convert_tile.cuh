@@ -22,7 +22,7 @@
 //
 // Work: items (product z, polynomial, column group cg); a tile holds
 // coefficient r*C + Gc*cg + c in row m = r*Gc + c (Gc = min(C, 8)), as in K1T.
-// Barriers: tma_full[2], mma_full, tmem_empty (256 arrivals), b_full.  Every
+// Barriers: tma_full[2], mma_full, tmem_empty (one arrival a warp), b_full.  Every
 // wait is bounded; a wait that gives up stops the CTA, lets its copies land,
 // frees the TMEM and sets the plan's error word.
 #pragma once
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) tc::mbar_init(&tma_full[b], 1);
         tc::mbar_init(&mma_full, 1);
-        tc::mbar_init(&tmem_empty, 256);
+        tc::mbar_init(&tmem_empty, 8);
         tc::mbar_init(&b_full, 1);
         s_abort = 0;
     }
@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
                 }
             }
             tc::fence_before();
-            tc::mbar_arrive(&tmem_empty);  // this thread's accumulator reads are complete
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&tmem_empty);  // this warp's accumulator reads are complete
             tc::bar_sync(1, 256);
             // --- forward column stages of (prime, column) pairs, then the residue planes ---
             const int pairs = tP * Gc;

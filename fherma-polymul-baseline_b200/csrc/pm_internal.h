@@ -40,12 +40,14 @@ struct DeviceBasis {
     int device = 0;
     std::vector<uint32_t> primes;   // kPMax primes, descending
     std::vector<uint32_t> inv1;     // [kPMax] psi^-brev(1): the inverse twiddle of the last column stage
+    std::vector<uint32_t> fwd8;     // [kPMax][8] psi^brev(k), k < 8: the first three column stages' twiddles
     PrimeConst* d_pc = nullptr;     // [kPMax]
     uint2* d_tw_fwd = nullptr;      // [kPMax][kNMax] psi^brev(k)   (value, Shoup)
     uint2* d_tw_inv = nullptr;      // [kPMax][kNMax] psi^-brev(k)
     uint2* d_conv_pow = nullptr;    // [kPMax][kPowWords] 2^(32k) mod p
     // tensor-core conversion table (built on first tensor plan)
     uint8_t* d_conv_weights = nullptr;
+    uint8_t* d_fold_weights = nullptr;  // [3][128 KB] weights with 1, 2 and 3 column stages folded in
     ~DeviceBasis();
 };
 

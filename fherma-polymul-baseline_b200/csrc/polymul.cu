@@ -208,6 +208,7 @@ DeviceBasis& basis_for_device(int device) {
     std::vector<PrimeConst> pc(P);
     std::vector<uint2> fwd(P * kNMax), inv(P * kNMax), pow(P * kPowWords);
     B->inv1.assign(P, 0);
+    B->fwd8.assign(P * 8, 0);
     auto fill = [&](size_t begin, size_t end) {
         for (size_t i = begin; i < end; ++i) {
             const uint32_t p = B->primes[i];
@@ -220,6 +221,7 @@ DeviceBasis& basis_for_device(int device) {
             }
             pc[i] = prime_const(p);
             B->inv1[i] = inv[i * kNMax + 1].x;
+            for (int k = 0; k < 8; ++k) B->fwd8[i * 8 + k] = fwd[i * kNMax + k].x;
         }
     };
     unsigned nt = std::thread::hardware_concurrency();

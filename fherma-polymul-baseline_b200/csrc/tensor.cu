@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -15,6 +16,7 @@
 #include "tc_ptx.cuh"
 #include "tensor_kernels.cuh"
 #include "convert_tile.cuh"
+#include "convert_fold.cuh"
 #include "crt_quartic.cuh"
 
 namespace pm {
@@ -42,6 +44,42 @@ std::vector<uint8_t> conversion_image(const std::vector<uint32_t>& primes) {
     }
     return img;
 }
+
+// K1F's weights for f folded column stages (convert_fold.cuh): [4 bytes a][2 K atoms][128 lanes][128 B].
+// Lane h (128 >> f) + i, K position h' (256 >> f) + k: byte a of T_i[h][h'] 2^(8k) mod p_i, T_i the f
+// forward butterfly stages over the 2^f row blocks.
+std::vector<uint8_t> fold_image(const DeviceBasis& B, int f) {
+    const int F = 1 << f, pmax = 128 >> f, span = 256 >> f;
+    std::vector<uint8_t> img(kFoldWeightBytes, 0);
+    for (int i = 0; i < pmax && i < int(B.primes.size()); ++i) {
+        const uint32_t p = B.primes[size_t(i)];
+        uint32_t T[8][8] = {};
+        for (int h = 0; h < F; ++h) T[h][h] = 1;
+        for (int s = 0; s < f; ++s) {
+            const int d = F >> (s + 1);
+            for (int h = 0; h < F; ++h) {
+                if (h & d) continue;
+                const uint32_t w = B.fwd8[size_t(i) * 8 + size_t(1 << s) + size_t(h >> (f - s))];
+                for (int g = 0; g < F; ++g) {
+                    const uint32_t x = T[h][g], y = uint32_t(uint64_t(T[h + d][g]) * w % p);
+                    T[h][g] = (x + y) % p;
+                    T[h + d][g] = (x + p - y) % p;
+                }
+            }
+        }
+        for (int h = 0; h < F; ++h)
+            for (int g = 0; g < F; ++g) {
+                uint32_t v = T[h][g];
+                for (int k = 0; k < span; ++k, v = uint32_t(uint64_t(v) * 256 % p)) {
+                    const int K = g * span + k;
+                    for (int a = 0; a < 4; ++a)
+                        img[size_t(a) * 32768 + size_t(K >> 7) * 16384 +
+                            tc::sw128_offset(uint32_t(h * pmax + i), uint32_t(K & 127))] = uint8_t(v >> (8 * a));
+                }
+            }
+    }
+    return img;
+}
 }  // namespace
 
 void tensor_init(PlanCore& s) {
@@ -57,6 +95,16 @@ void tensor_init(PlanCore& s) {
             cuda_check(cudaMalloc(&B.d_conv_weights, img.size()), "allocate conversion weights");
             cuda_check(cudaMemcpy(B.d_conv_weights, img.data(), img.size(), cudaMemcpyHostToDevice),
                        "upload conversion weights");
+        }
+        if (!B.d_fold_weights) {
+            std::vector<uint8_t> fold;
+            for (int f = 1; f <= 3; ++f) {
+                const auto one = fold_image(B, f);
+                fold.insert(fold.end(), one.begin(), one.end());
+            }
+            cuda_check(cudaMalloc(&B.d_fold_weights, fold.size()), "allocate folded conversion weights");
+            cuda_check(cudaMemcpy(B.d_fold_weights, fold.data(), fold.size(), cudaMemcpyHostToDevice),
+                       "upload folded conversion weights");
         }
     }
     // CRT weights: [2 K-atoms][128 rows][128 B].  Row (i, a) holds the bytes of
@@ -226,11 +274,70 @@ void launch_k1w(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
     kernel<<<ctas, tc::kWideThreads, smem, st>>>(w, s.plane_pc(), s.conv_weights(), s.plane_fwd(), s.d_err, fix);
 }
 
+// Coefficient bytes for K1F: boxes of the row block's (256 >> f) bytes x 2^(f + 3) columns x 16 >> f rows.
+CUtensorMap fold_map(const PlanCore& s, const void* base, uint32_t count, int f) {
+    const uint32_t C = 1u << s.logC, R = 16;
+    const cuuint64_t sb = s.stride * 4ull;
+    const cuuint64_t dims[4] = {sb, C, R, count};
+    const cuuint64_t strides[3] = {sb, sb * C, sb * C * R};
+    const cuuint32_t box[4] = {256u >> f, 8u << f, 16u >> f, 1};
+    const CUtensorMapSwizzle swizzle = f == 1 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                              : (f == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+    return make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, base, dims, strides, box, swizzle);
+}
+
+// folded stages of this plan's conversion by K1F, or 0 where it does not apply: the quartic
+// factorization's own weights, views of fewer than 16 rows
+int plan_fold(const PlanCore& s) {
+    return s.quartic || s.logR != 4 ? 0 : fold_stages(int(s.P), int(s.logC));
+}
+
+template <int LOGF>
+void launch_k1f(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
+                cudaStream_t st, int poly_only) {
+    PlanFoldWork w;
+    w.poly_only = poly_only;
+    w.map_a = fold_map(s, poly_only == 1 ? b : a, count, LOGF);
+    w.map_b = poly_only == 0 ? w.map_a : fold_map(s, b, count, LOGF);
+    w.work = work;
+    w.ws_bstride = s.workspace_bytes / 4;
+    w.n = int(s.n);
+    w.logC = int(s.logC);
+    w.P = int(s.P);
+    w.count = int(count);
+    w.log_groups = int(s.logC) - (LOGF + 3);
+    const int items = int(count) * (poly_only < 0 ? 2 : 1) << w.log_groups;
+    auto kernel = k1f_convert<LOGF, PlanFoldWork>;
+    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k1f_smem_bytes())),
+               "K1F shared memory");
+    kernel<<<std::min(items, s.sms), kFoldThreads, k1f_smem_bytes(), st>>>(
+        w, s.basis->d_pc, s.basis->d_fold_weights + (LOGF - 1) * size_t(kFoldWeightBytes), s.basis->d_tw_fwd,
+        int((s.qbits + 7) / 8), s.d_err);
+}
+
+// Conversion of both polynomials (poly_only < 0) or of one, by the folding kernel or K1W.  K1F
+// loads 128 KB of weights per CTA before its first tile, against K1W's 32 KB and twice the CTAs:
+// K1W stays where it finishes in two rounds (592 tiles of 128 coefficients on 148 SMs).  Measured
+// on either side, whole products (868 bits unless said): n = 32768, one 38.8 us by K1W / 39.2 by
+// K1F, two 64.6 / 64.3, eight 189.7 / 183.9; n = 1024, one 17.1 / 19.4, 32 of 200 bits (512 tiles)
+// 19.5 / 20.0; n = 4096, 16 of 200 bits (1024 tiles) 27.4 / 25.0.
+template <int LOGR>
+void launch_whole_basis(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
+                        cudaStream_t st, int poly_only = -1) {
+    const size_t tiles = size_t(count) * (poly_only < 0 ? 2 : 1) * s.n / tc::kTileM;
+    switch (LOGR == 4 && tiles > size_t(s.sms) * 4 ? plan_fold(s) : 0) {
+        case 1: return launch_k1f<1>(s, a, b, work, count, st, poly_only);
+        case 2: return launch_k1f<2>(s, a, b, work, count, st, poly_only);
+        case 3: return launch_k1f<3>(s, a, b, work, count, st, poly_only);
+        default: return launch_k1w<LOGR>(s, a, b, work, count, st, poly_only);
+    }
+}
+
 template <int LOGR>
 void launch_conversion(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
                        cudaStream_t st) {
     if (s.tune.conv_whole_basis)
-        launch_k1w<LOGR>(s, a, b, work, count, st);
+        launch_whole_basis<LOGR>(s, a, b, work, count, st);
     else
         launch_k1t<LOGR>(s, a, b, work, count, st);
 }
@@ -361,11 +468,11 @@ void launch_tensor_convert_poly(const PlanCore& s, const uint32_t* x, int poly, 
     const uint32_t* a = poly == 0 ? x : nullptr;
     const uint32_t* b = poly == 1 ? x : nullptr;
     switch (s.logR) {
-        case 0: launch_k1w<0>(s, a, b, work, 1, st, poly); break;
-        case 1: launch_k1w<1>(s, a, b, work, 1, st, poly); break;
-        case 2: launch_k1w<2>(s, a, b, work, 1, st, poly); break;
-        case 3: launch_k1w<3>(s, a, b, work, 1, st, poly); break;
-        default: launch_k1w<4>(s, a, b, work, 1, st, poly); break;
+        case 0: launch_whole_basis<0>(s, a, b, work, 1, st, poly); break;
+        case 1: launch_whole_basis<1>(s, a, b, work, 1, st, poly); break;
+        case 2: launch_whole_basis<2>(s, a, b, work, 1, st, poly); break;
+        case 3: launch_whole_basis<3>(s, a, b, work, 1, st, poly); break;
+        default: launch_whole_basis<4>(s, a, b, work, 1, st, poly); break;
     }
     cuda_check(cudaGetLastError(), "launch conversion");
     count_launches(1);

@@ -103,8 +103,9 @@ typedef struct {
                                    of >= 1024 values: one CTA each, prefetched; of 16 .. 512: a warp per 512
                                    values, row_radix unused); 0: CTAs per row, twiddles read per product */
     uint32_t conv_whole_basis;  /* tensor conversion: 1 (the default) takes each coefficient tile through all
-                                   primes at once (weights of the whole basis resident, 2 CTAs per SM;
-                                   conv_ctas_per_sm unused); 0 runs it once per group of 16 primes */
+                                   primes at once (conv_ctas_per_sm unused; launches of more than four tiles
+                                   an SM also fold column stages into the contraction); 0 runs it once per
+                                   group of 16 primes */
     double us_per_product;      /* device time the autotuner measured (-1: taken from its cache) */
 } pm_tuning;
 
