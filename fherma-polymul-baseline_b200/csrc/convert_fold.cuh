@@ -23,15 +23,18 @@
 // M = 128, K = 32 MMA takes 60 cycles at any N up to 64 and 64 at N = 128.  The accumulators of
 // bytes 0 and 1 and of bytes 2 and 3 are two buffers: while the epilogue folds one pair into
 // registers the MMAs fill the other, of this tile or the next.  A producer warp issues loads
-// and MMAs; kFoldSets sets of four warps (the 128 TMEM lanes) take half tiles (half the columns)
+// and MMAs (a warp of its own for the loads measured 5% slower); kFoldSets sets of four warps (the 128 TMEM lanes) take half tiles (half the columns)
 // in turn, so one set's stages and stores overlap another's accumulator reads.
 // Measured: 6.98 -> 5.60 us a product (868 bits, n = 32768, 128 products), 3.13 -> 2.72 us at
 // n = 16384 (640 bits), 2.05 -> 1.53 us at n = 8192.  At 32768 it issues 21 instructions a residue
 // (K1W 30) and moves 22.8 MB in 5.6 us (4.1 TB/s); left are the multiply pipe (62%), the 32-byte
 // stores (each touches its own line: 32 lines an instruction; 16-byte ones cost 0.2 ms more) and
 // the chain MMA - accumulator read - stages of few warps (three sets of 128 registers; two
-// of 168 and four of 96 measured 1-2% and 23% slower).
-// Barriers: tma_full[3]; full[set][pair] (an accumulator pair is complete) and done[2] (the
+// of 168 and four of 96 measured 1-2% and 23% slower).  The form without tensor maps converts 60
+// products of 517 bits (9 limbs, n = 4096) in 64 us against 54 for the same with 10 limbs by TMA
+// (one loader warp 99, two 70); copying rows of even limbs 16 bytes at a time instead of by
+// TMA measured 6% to 13% slower.
+// Barriers: tma_full[3]; full[set][pair] (an accumulator pair is complete) and done[3] (the
 // tile's buffer is free), from MMA commits; empty[pair] (one arrival a warp: the pair has been
 // read); w_full.  Every wait is bounded; one that gives up stops the CTA, lets its
 // copies land, frees the TMEM and sets the plan's error word.
@@ -42,7 +45,7 @@
 namespace pm {
 
 constexpr int kFoldSets = 3;
-constexpr int kFoldThreads = 32 * (4 * kFoldSets + 1);
+constexpr int kFoldLoaders = 3;                  // loader warps of the form without tensor maps
 constexpr int kFoldTiles = 3;                    // coefficient tiles in flight
 constexpr int kFoldTileBytes = 32768;            // 128 rows of 256 bytes
 constexpr uint32_t kFoldWeightBytes = 4 * 32768;  // 4 bytes a, 128 rows, K = 256
@@ -64,6 +67,7 @@ struct PlanFoldWork {
     size_t ws_bstride;
     int n, logC, P, count;
     int poly_only, log_groups;  // column groups per row = 2^log_groups
+    PlainRows plain;            // (the form that loads rows without tensor maps)
     __device__ int total() const { return count << (log_groups + (poly_only < 0 ? 1 : 0)); }
     __device__ TileItem item(int k) const {
         const int g = log_groups, cg = k & ((1 << g) - 1);
@@ -108,9 +112,13 @@ __device__ __forceinline__ void store8(uint32_t* p, const uint32_t (&v)[8], bool
     }
 }
 
+constexpr int k1f_threads(bool plain) { return 32 * (4 * kFoldSets + 1 + (plain ? kFoldLoaders : 0)); }
+
 // LOGF: folded stages f.  qbytes: bytes a coefficient can have (K steps past them are skipped).
-template <int LOGF, class Work>
-__global__ void __launch_bounds__(kFoldThreads, 1)
+// PLAIN: coefficient rows a tensor map cannot describe (w.plain); kFoldLoaders more warps copy
+// them into the same swizzled layout, 8 bytes at a time, a tile ahead of the one they hand over.
+template <int LOGF, class Work, bool PLAIN = false>
+__global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
     k1f_convert(const __grid_constant__ Work w, const PrimeConst* __restrict__ pcs, const uint8_t* __restrict__ weights,
                 const uint2* __restrict__ tw_fwd, int qbytes, uint32_t* __restrict__ err) {
     constexpr int F = 1 << LOGF, J = 16 >> LOGF, PMAX = 128 >> LOGF;
@@ -122,7 +130,7 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
     uint8_t* sbase = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sW = sbase;                     // [4][2][128 rows x 128 B]
     uint8_t* sX = sbase + kFoldWeightBytes;  // [kFoldTiles][F][128 rows x SPAN B]
-    __shared__ uint64_t tma_full[kFoldTiles], full[kFoldSets][2], done[2], empty[2], w_full;
+    __shared__ uint64_t tma_full[kFoldTiles], full[kFoldSets][2], done[kFoldTiles], empty[2], w_full;
     __shared__ uint32_t tmem_base;
     __shared__ volatile uint32_t s_abort;
 
@@ -131,12 +139,17 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
     const int begin = int(int64_t(blockIdx.x) * total / gridDim.x);
     const int tiles = int(int64_t(blockIdx.x + 1) * total / gridDim.x) - begin;
 
+    if constexpr (PLAIN)  // the bytes past the copied words stay zero
+        for (int k = tid; k < kFoldTiles * kFoldTileBytes / 16; k += k1f_threads(PLAIN))
+            reinterpret_cast<uint4*>(sX)[k] = make_uint4(0, 0, 0, 0);
     if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
     if (tid == 0) {
-        for (int b = 0; b < kFoldTiles; ++b) tc::mbar_init(&tma_full[b], 1);
+        for (int b = 0; b < kFoldTiles; ++b) {
+            tc::mbar_init(&tma_full[b], PLAIN ? 32 * kFoldLoaders : 1);
+            tc::mbar_init(&done[b], 1);
+        }
         for (int b = 0; b < 2; ++b) {
             for (int g = 0; g < kFoldSets; ++g) tc::mbar_init(&full[g][b], 1);
-            tc::mbar_init(&done[b], 1);
             tc::mbar_init(&empty[b], 8);
         }
         tc::mbar_init(&w_full, 1);
@@ -150,7 +163,7 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
     bool ok = true;
 
     if (warp == 4 * kFoldSets) {
-        // ------------------------------ producer ------------------------------
+        // --------------------- MMAs (and the tiles' TMA loads) ----------------
         auto issue = [&](int kk) {
             const TileItem it = w.item(begin + kk);
             const ConvTarget t = w.target(it.z, it.poly);
@@ -171,12 +184,13 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
                 tc::mbar_expect_tx(&w_full, kFoldWeightBytes);
                 for (uint32_t o = 0; o < kFoldWeightBytes; o += 32768) tc::bulk_load(sW + o, weights + o, 32768u, &w_full);
             }
-            for (; issued < kFoldTiles && issued < tiles; ++issued)
-                if (lane == 0) issue(issued);
+            if (!PLAIN)
+                for (; issued < kFoldTiles && issued < tiles; ++issued)
+                    if (lane == 0) issue(issued);
             w_pending = !wait(&w_full, 0);
         }
         for (int kk = 0; kk < tiles && ok; ++kk) {
-            if (__any_sync(0xffffffffu, s_abort != 0)) break;  // an epilogue gave up a wait
+            if (__any_sync(0xffffffffu, s_abort != 0)) break;  // another warp gave up a wait
             const int b = kk % kFoldTiles;
             if (!wait(&tma_full[b], uint32_t(kk / kFoldTiles) & 1u)) break;
             ++seen;
@@ -198,15 +212,15 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
                         }
                     tc::mma_commit(&full[(2 * kk) % kFoldSets][pair]);  // the sets of the tile's halves
                     tc::mma_commit(&full[(2 * kk + 1) % kFoldSets][pair]);
-                    if (pair) tc::mma_commit(&done[kk & 1]);
+                    if (pair) tc::mma_commit(&done[b]);
                 }
                 __syncwarp();
             }
             if (!ok) break;
             ++committed;
             // the previous tile's MMAs have read its buffer: it takes the next tile to request
-            if (kk >= 1) {
-                if (!wait(&done[(kk - 1) & 1], uint32_t((kk - 1) >> 1) & 1u)) break;
+            if (!PLAIN && kk >= 1) {
+                if (!wait(&done[(kk - 1) % kFoldTiles], uint32_t((kk - 1) / kFoldTiles) & 1u)) break;
                 if (issued < tiles) {
                     if (lane == 0) issue(issued);
                     ++issued;
@@ -218,7 +232,51 @@ __global__ void __launch_bounds__(kFoldThreads, 1)
         // last MMAs complete before it frees the tensor memory
         for (; seen < issued; ++seen) tc::mbar_wait(&tma_full[seen % kFoldTiles], uint32_t(seen / kFoldTiles) & 1u);
         if (w_pending) tc::mbar_wait(&w_full, 0);
-        if (committed) tc::mbar_wait(&done[(committed - 1) & 1], uint32_t((committed - 1) >> 1) & 1u);
+        if (committed)
+            tc::mbar_wait(&done[(committed - 1) % kFoldTiles], uint32_t((committed - 1) / kFoldTiles) & 1u);
+    } else if (PLAIN && warp > 4 * kFoldSets) {
+        // ------------------------------ loaders -------------------------------
+        if constexpr (PLAIN) {
+            constexpr int T = 32 * kFoldLoaders;
+            const int words = w.plain.copied;
+            const int t0 = tid - k1f_threads(false);
+            const int step_r = T / words, step_w = T - step_r * words;
+            auto hand_over = [&](int kk) {  // this thread's copies of tile kk have landed
+                tc::fence_smem_async();
+                tc::mbar_arrive(&tma_full[kk % kFoldTiles]);
+            };
+            int loaded = 0;
+            for (int kk = 0; kk < tiles; ++kk, ++loaded) {
+                const int b = kk % kFoldTiles;
+                if (kk >= kFoldTiles)  // the MMAs have read the buffer's last tile
+                    ok = tc::mbar_wait(&done[b], uint32_t(kk / kFoldTiles - 1) & 1u) && ok;
+                if (__any_sync(0xffffffffu, !ok || s_abort)) break;
+                const TileItem it = w.item(begin + kk);
+                const ConvTarget t = w.target(it.z, it.poly);
+                // row r of the tile: block r >> 7, then (row, column) n = r & 127; words in order
+                int r = t0 / words, wd = t0 - r * words;
+                while (r < 128 * F) {
+                    const int n = r & 127, coef = (((r >> 7) * J + n / COLS) << t.logC) + it.cg * COLS + n % COLS;
+                    const uint32_t off = uint32_t(n * SPAN + 8 * wd);
+                    tc::cp_async8(sX + b * kFoldTileBytes + (r >> 7) * BOX + (off ^ (((off >> 7) & (SPAN / 16 - 1)) << 4)),
+                                  w.plain.row(it.z, it.poly, t.n, coef) + wd);
+                    r += step_r;
+                    wd += step_w;
+                    if (wd >= words) {
+                        wd -= words;
+                        ++r;
+                    }
+                }
+                tc::cp_async_commit();
+                if (kk >= 1) {
+                    tc::cp_async_wait<1>();
+                    hand_over(kk - 1);
+                }
+            }
+            tc::cp_async_wait<0>();
+            if (loaded) hand_over(loaded - 1);
+            if (!ok) s_abort = 1;
+        }
     } else {
         // ------------------------------ epilogue ------------------------------
         const int set = warp >> 2;

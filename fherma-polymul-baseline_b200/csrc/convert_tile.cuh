@@ -40,6 +40,18 @@ struct TileItem {
     int z, poly, cg;
 };
 
+// Coefficients of a, b as rows of `words` u64 (of which the first `copied` can be non-zero),
+// for layouts a tensor map cannot describe: an odd number of limbs makes a row pitch that is
+// not a multiple of 16 bytes.
+struct PlainRows {
+    const uint64_t* x[2];
+    int words, copied;
+    // row `coef` of polynomial `poly` of product z
+    __device__ const uint64_t* row(int z, int poly, int n, int coef) const {
+        return x[poly] + (size_t(z) * n + coef) * words;
+    }
+};
+
 // `count` products of one plan: items (z, poly, cg) numbered product-major; with
 // poly_only = 0 or 1, the items of that polynomial alone (its conversion can start
 // while the other polynomial is still arriving).
@@ -49,6 +61,7 @@ struct PlanTileWork {
     size_t ws_bstride;
     int n, logC, P, count;
     int poly_only;  // -1: both polynomials
+    PlainRows plain;  // (kernels that load rows without tensor maps)
     __device__ int lg() const { return logC - min(logC, 3); }  // column groups per row = 2^lg
     __device__ int total() const { return count << (lg() + (poly_only < 0 ? 1 : 0)); }
     __device__ TileItem item(int k) const {
@@ -73,7 +86,9 @@ constexpr size_t k1w_smem_bytes() { return 1024 + 32768 + 32768 + size_t(tc::kMa
 
 // LOGC > 0: every item's rows hold 2^LOGC values (a plan's launch at a common ring size),
 // so row strides and plane offsets are constants; 0: read from the item.
-template <int LOGR, class Work, int LOGC = 0>
+// PLAIN: coefficient rows without a tensor map (w.plain): the producer warp copies a tile's
+// rows with 8-byte asynchronous copies into the same swizzled layout (rows of 8 columns or more).
+template <int LOGR, class Work, int LOGC = 0, bool PLAIN = false>
 __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_constant__ Work w,
                                                                     const PrimeConst* __restrict__ pcs,
                                                                     const uint8_t* __restrict__ conv_w,
@@ -128,8 +143,25 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
             const TileItem it = w.item(k);
             const ConvTarget t = w.target(it.z, it.poly);
             const int C = 1 << (LOGC ? LOGC : t.logC), Gc = C < 8 ? C : 8;
-            tc::mbar_expect_tx(&tma_full[buf], 128u * uint32_t(Gc) * uint32_t(R));
-            tc::tma_load_4d(sA + buf * 16384, t.map, 0, it.cg * Gc, 0, t.mz, &tma_full[buf]);
+            if constexpr (PLAIN) {  // by the whole warp: words in order, so a run of 8 rows is one stretch
+                const int words = w.plain.copied;
+                const int step_m = 32 / words, step_w = 32 - step_m * words;
+                int m = lane / words, wd = lane - m * words;
+                while (m < 8 * R) {
+                    tc::cp_async8(sA + buf * 16384 + tc::sw128_offset(m, 8 * wd),
+                                  w.plain.row(it.z, it.poly, t.n, ((m >> 3) << t.logC) + it.cg * 8 + (m & 7)) + wd);
+                    m += step_m;
+                    wd += step_w;
+                    if (wd >= words) {
+                        wd -= words;
+                        ++m;
+                    }
+                }
+                tc::cp_async_commit();
+            } else {
+                tc::mbar_expect_tx(&tma_full[buf], 128u * uint32_t(Gc) * uint32_t(R));
+                tc::tma_load_4d(sA + buf * 16384, t.map, 0, it.cg * Gc, 0, t.mz, &tma_full[buf]);
+            }
         };
         auto wait = [&](uint64_t* bar, uint32_t parity) {
             const bool done = __all_sync(0xffffffffu, tc::mbar_wait(bar, parity));
@@ -141,6 +173,8 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
         if (lane == 0 && begin < end) {
             tc::mbar_expect_tx(&b_full, 32768u);
             tc::bulk_load(sB, conv_w, 32768u, &b_full);
+        }
+        if ((PLAIN || lane == 0) && begin < end) {
             issue(begin, 0);
             if (begin + 1 < end) issue(begin + 1, 1);
         }
@@ -153,9 +187,18 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
         for (int k = begin; k < end && ok; ++k, ++kk) {
             if (__any_sync(0xffffffffu, s_abort != 0)) break;  // a worker gave up a wait
             const int buf = kk & 1;
-            if (!wait(&tma_full[buf], (ph_tma >> buf) & 1u)) break;
-            ph_tma ^= 1u << buf;
-            pending &= ~(1u << buf);
+            if constexpr (PLAIN) {  // the tile before the newest group, or the last one
+                if (k + 1 < end)
+                    tc::cp_async_wait<1>();
+                else
+                    tc::cp_async_wait<0>();
+                tc::fence_smem_async();
+                __syncwarp();
+            } else {
+                if (!wait(&tma_full[buf], (ph_tma >> buf) & 1u)) break;
+                ph_tma ^= 1u << buf;
+                pending &= ~(1u << buf);
+            }
             if (kk >= 1) {  // the workers have read the previous tile's accumulator
                 if (!wait(&tmem_empty, ph_empty)) break;
                 ph_empty ^= 1u;
@@ -185,14 +228,17 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
             if (!wait(&mma_full, ph_mma)) break;
             ph_mma ^= 1u;
             if (k + 2 < end) {
-                if (lane == 0) issue(k + 2, buf);
+                if (PLAIN || lane == 0) issue(k + 2, buf);
                 pending |= 1u << buf;
             }
         }
         if (!ok) s_abort = 1;
         // copies requested but not consumed land before the CTA's shared memory goes away
-        for (int b = 0; b < 2; ++b)
-            if (pending & (1u << b)) tc::mbar_wait(&tma_full[b], (ph_tma >> b) & 1u);
+        if constexpr (PLAIN)
+            tc::cp_async_wait<0>();
+        else
+            for (int b = 0; b < 2; ++b)
+                if (pending & (1u << b)) tc::mbar_wait(&tma_full[b], (ph_tma >> b) & 1u);
         if (b_pending) tc::mbar_wait(&b_full, 0);
     } else {
         // ------------------------------ workers -------------------------------

@@ -109,7 +109,7 @@ void* fherma_init(const fherma::Point& p) {
     s->words = p.L;
     const uint32_t limbs = p.L / 2;
     // the tensor-core conversion reads 16-byte coefficient rows (even limb counts)
-    const uint32_t flags = (limbs % 2 == 0) ? PM_CONVERT_TENSOR : PM_CONVERT_SIMT;
+    const uint32_t flags = (limbs % 2 == 0) ? PM_CONVERT_TENSOR : PM_CONVERT_DEFAULT;
     const int st = pm_plan_create(&s->plan, p.N, q64.data(), limbs, limbs, flags);
     if (st != PM_OK) raise(st, "fherma_init");
     s->spare = std::make_unique<SpareOutput>(size_t(p.N) * p.L);

@@ -138,22 +138,68 @@ inline Words shift_left(const Words& a, unsigned bits) {
     return r;
 }
 
-// floor(x / q) and x mod q by binary long division (set-up only).
+// floor(x / q) and x mod q by schoolbook long division, a word of quotient at a time
+// (Knuth, The Art of Computer Programming 2, 4.3.1, algorithm D).
 inline void divmod(const Words& x, const Words& q, Words* quotient, Words* remainder) {
-    unsigned xb = bit_length(x);
-    Words rem;
-    Words quo((xb + 31) / 32 + 1, 0);
-    for (unsigned bit = xb; bit--;) {
-        rem = shift_left(rem, 1);
-        if ((x[bit / 32] >> (bit % 32)) & 1) {
-            if (rem.empty()) rem.push_back(0);
-            rem[0] |= 1;
+    Words d = q;
+    trim(d);
+    if (d.empty()) throw std::logic_error("multiprecision division by zero");
+    Words quo, rem;
+    if (compare(x, d) < 0) {
+        rem = x;
+    } else if (d.size() == 1) {
+        quo = x;
+        const uint32_t r = divide_small(quo, d[0]);
+        rem.assign(1, r);
+    } else {
+        const size_t n = d.size();
+        const unsigned sh = unsigned(__builtin_clz(d[n - 1]));
+        d = shift_left(d, sh);
+        Words u = shift_left(x, sh);
+        u.resize((x.size() > u.size() ? x.size() : u.size()) + 1, 0);
+        const size_t m = u.size() - n;  // quotient words
+        quo.assign(m, 0);
+        for (size_t j = m; j--;) {
+            // the estimate from the top words is at most two too large once refined
+            const uint64_t top = (uint64_t(u[j + n]) << 32) | u[j + n - 1];
+            uint64_t qhat, rhat;
+            if (u[j + n] >= d[n - 1]) {
+                qhat = 0xffffffffull;
+                rhat = top - qhat * d[n - 1];
+            } else {
+                qhat = top / d[n - 1];
+                rhat = top % d[n - 1];
+            }
+            while (rhat <= 0xffffffffull && qhat * d[n - 2] > ((rhat << 32) | u[j + n - 2])) {
+                --qhat;
+                rhat += d[n - 1];
+            }
+            uint64_t carry = 0, borrow = 0;
+            for (size_t i = 0; i < n; ++i) {
+                const uint64_t prod = qhat * d[i] + carry;
+                carry = prod >> 32;
+                const uint64_t sub = uint64_t(u[i + j]) - uint32_t(prod) - borrow;
+                u[i + j] = uint32_t(sub);
+                borrow = sub >> 63;
+            }
+            const uint64_t sub = uint64_t(u[j + n]) - carry - borrow;
+            u[j + n] = uint32_t(sub);
+            if (sub >> 63) {  // one too large: add the divisor back
+                --qhat;
+                uint64_t c = 0;
+                for (size_t i = 0; i < n; ++i) {
+                    c += uint64_t(u[i + j]) + d[i];
+                    u[i + j] = uint32_t(c);
+                    c >>= 32;
+                }
+                u[j + n] += uint32_t(c);
+            }
+            quo[j] = uint32_t(qhat);
         }
-        if (compare(rem, q) >= 0) {
-            rem = subtract(rem, q);
-            trim(rem);
-            quo[bit / 32] |= 1u << (bit % 32);
-        }
+        u.resize(n);
+        rem.assign(n, 0);
+        for (size_t i = 0; i < n; ++i)
+            rem[i] = sh ? (u[i] >> sh) | (i + 1 < n ? u[i + 1] << (32 - sh) : 0) : u[i];
     }
     trim(quo);
     trim(rem);

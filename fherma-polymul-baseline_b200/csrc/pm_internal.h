@@ -138,6 +138,7 @@ struct PlanCore {
     uint32_t W = 0;          // q words rounded up to a multiple of 4 (kernel template width)
     uint32_t coef_limbs = 0, stride = 0;  // u64 limbs and u32 words per coefficient
     uint32_t flags = 0;
+    bool plain_rows = false;  // tensor path over an odd coef_limbs: coefficient rows loaded without tensor maps
     Words q;
     uint64_t mu_q = 0;
     uint32_t delta = 0;      // q = 2^qbits - delta, delta < 2^32, PM_SPECIAL_FORM asked: folding reduction; else 0
@@ -189,8 +190,8 @@ void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t
 void check_device_errors(const PlanCore& s);
 // Device-pointer arguments a kernel may touch: reachable from the device (not
 // pageable host memory), 8-byte aligned (u64 coefficients; the kernels move 8
-// and 16 bytes at a time), and 16-byte aligned on the tensor path (tensor maps
-// of a, b and the residue workspace).  Throws PM_ERR_INVALID otherwise.
+// and 16 bytes at a time), and 16-byte aligned on the tensor path of an even
+// coef_limbs (tensor maps of a, b and the residue workspace).  Throws PM_ERR_INVALID otherwise.
 void check_device_pointers(const PlanCore& s, const void* a, const void* b, const void* c, const void* workspace);
 // Calls on device pointers run on the caller's current device, which must be the
 // plan's: its tables, twiddles, error word and workspace live there.  Throws

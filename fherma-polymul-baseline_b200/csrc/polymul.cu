@@ -297,9 +297,14 @@ void PlanCore::init(uint32_t n_, const uint64_t* q64, uint32_t q_limbs, uint32_t
         throw Failure(PM_ERR_INVALID, "PM_QUARTIC runs on the tensor path only");
     if ((flags_ & PM_CONVERT_TENSOR) && (flags_ & PM_CONVERT_SIMT))
         throw Failure(PM_ERR_INVALID, "PM_CONVERT_TENSOR and PM_CONVERT_SIMT exclude each other");
-    // no path asked for: the tensor path wherever its 16-byte coefficient rows exist
-    if (!(flags_ & (PM_CONVERT_TENSOR | PM_CONVERT_SIMT | PM_WIDE_NTT)) && coef_limbs_ % 2 == 0)
+    // No path asked for: the tensor path, over an odd coef_limbs (row pitches a tensor map cannot
+    // describe) by the conversion kernels' plain-row forms, which take rows of 16 columns or more
+    // (n >= 256).  60 products of 517 bits (9 limbs) at n = 4096: 396 us by the plain method, 135 us so.
+    plain_rows = false;
+    if (!(flags_ & (PM_CONVERT_TENSOR | PM_CONVERT_SIMT | PM_WIDE_NTT)) && (coef_limbs_ % 2 == 0 || n_ >= 256)) {
         flags_ |= PM_CONVERT_TENSOR;
+        plain_rows = coef_limbs_ % 2 != 0;
+    }
     q.assign(2 * q_limbs, 0);
     for (uint32_t i = 0; i < q_limbs; ++i) {
         q[2 * i] = uint32_t(q64[i]);
@@ -583,7 +588,7 @@ void check_device_pointers(const PlanCore& s, const void* a, const void* b, cons
         if (!ptrs[i]) continue;
         const uintptr_t addr = reinterpret_cast<uintptr_t>(ptrs[i]);
         // tensor path: tensor maps over a, b and the workspace; wide NTT: 16-byte workspace loads
-        const bool tensor = (s.flags & PM_CONVERT_TENSOR) != 0;
+        const bool tensor = (s.flags & PM_CONVERT_TENSOR) != 0 && !s.plain_rows;
         const uintptr_t need = (tensor && i != 2) || (s.wide && i == 3) ? 16 : 8;
         if (addr % need)
             throw Failure(PM_ERR_INVALID, std::string(names[i]) + " must be " + std::to_string(need) +

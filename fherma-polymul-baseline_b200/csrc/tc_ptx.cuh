@@ -156,6 +156,17 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
+// 8-byte asynchronous copy global -> shared by one thread (both addresses 8-byte aligned);
+// committed in groups, waited for by the thread that issued it
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
 // byte offset of (row m, byte k < 128) inside one 128-byte-swizzled atom column
 __host__ __device__ __forceinline__ uint32_t sw128_offset(uint32_t m, uint32_t k) {
     return (m >> 3) * 1024 + (m & 7) * 128 + ((((k >> 4) ^ (m & 7)) & 7) << 4) + (k & 15);

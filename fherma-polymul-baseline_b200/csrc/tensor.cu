@@ -85,7 +85,8 @@ std::vector<uint8_t> fold_image(const DeviceBasis& B, int f) {
 void tensor_init(PlanCore& s) {
     if (uint32_t(s.P) * 4 > uint32_t(tc::kCrtK)) throw Failure(PM_ERR_UNSUPPORTED, "prime basis too large for the CRT tile");
     if (4 * s.W + 16 > uint32_t(tc::kCrtN)) throw Failure(PM_ERR_UNSUPPORTED, "q too wide for the CRT tile");
-    if (s.stride % 4) throw Failure(PM_ERR_UNSUPPORTED, "tensor path needs an even coef_limbs (16-byte coefficient rows)");
+    if (s.stride % 4 && !s.plain_rows)
+        throw Failure(PM_ERR_UNSUPPORTED, "tensor path needs an even coef_limbs (16-byte coefficient rows)");
     DeviceBasis& B = *s.basis;
     {
         static std::mutex m;
@@ -237,6 +238,13 @@ void launch_k1t(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
                                                                            s.plane_fwd(), s.d_err);
 }
 
+// coefficient rows of an odd number of limbs: the words that fit `span` bytes can be non-zero
+PlainRows plain_rows(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t span) {
+    const uint32_t words = s.stride / 2, used = uint32_t(s.qbits + 63) / 64;
+    return PlainRows{{reinterpret_cast<const uint64_t*>(a), reinterpret_cast<const uint64_t*>(b)}, int(words),
+                     int(std::min(used, span / 8))};
+}
+
 // the whole basis per tile: two CTAs per SM, contiguous runs of items
 template <int LOGR>
 void launch_k1w(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
@@ -248,15 +256,21 @@ void launch_k1w(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
     const size_t smem = k1w_smem_bytes();
     // rows of 1024, 2048 or 4096 values (n = 16384 .. 65536): a kernel with that row length built in
     auto kernel = k1w_convert<LOGR, PlanTileWork>;
-    if (LOGR == 4 && s.logC == 10) kernel = k1w_convert<LOGR, PlanTileWork, 10>;
-    if (LOGR == 4 && s.logC == 11) kernel = k1w_convert<LOGR, PlanTileWork, 11>;
-    if (LOGR == 4 && s.logC == 12) kernel = k1w_convert<LOGR, PlanTileWork, 12>;
+    if constexpr (LOGR == 4)
+        if (s.plain_rows) kernel = k1w_convert<LOGR, PlanTileWork, 0, true>;
+    if (LOGR == 4 && s.logC == 10 && !s.plain_rows) kernel = k1w_convert<LOGR, PlanTileWork, 10>;
+    if (LOGR == 4 && s.logC == 11 && !s.plain_rows) kernel = k1w_convert<LOGR, PlanTileWork, 11>;
+    if (LOGR == 4 && s.logC == 12 && !s.plain_rows) kernel = k1w_convert<LOGR, PlanTileWork, 12>;
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
                "K1W shared memory");
     PlanTileWork w;
     w.poly_only = poly_only;
-    w.map_a = coefficient_map(s, poly_only == 1 ? b : a, count);
-    w.map_b = poly_only == 0 ? w.map_a : coefficient_map(s, b, count);
+    if (s.plain_rows) {
+        w.plain = plain_rows(s, a, b, 128);
+    } else {
+        w.map_a = coefficient_map(s, poly_only == 1 ? b : a, count);
+        w.map_b = poly_only == 0 ? w.map_a : coefficient_map(s, b, count);
+    }
     w.work = work;
     w.ws_bstride = s.workspace_bytes / 4;
     w.n = int(s.n);
@@ -287,9 +301,10 @@ CUtensorMap fold_map(const PlanCore& s, const void* base, uint32_t count, int f)
 }
 
 // folded stages of this plan's conversion by K1F, or 0 where it does not apply: the quartic
-// factorization's own weights, views of fewer than 16 rows
-int plan_fold(const PlanCore& s) {
-    return s.quartic || s.logR != 4 ? 0 : fold_stages(int(s.P), int(s.logC));
+// factorization's own weights, views of fewer than 16 rows, residue planes its 16-byte stores
+// cannot take (only plans of odd coef_limbs accept such a workspace)
+int plan_fold(const PlanCore& s, const uint32_t* work) {
+    return s.quartic || s.logR != 4 || reinterpret_cast<uintptr_t>(work) % 16 ? 0 : fold_stages(int(s.P), int(s.logC));
 }
 
 template <int LOGF>
@@ -297,8 +312,12 @@ void launch_k1f(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
                 cudaStream_t st, int poly_only) {
     PlanFoldWork w;
     w.poly_only = poly_only;
-    w.map_a = fold_map(s, poly_only == 1 ? b : a, count, LOGF);
-    w.map_b = poly_only == 0 ? w.map_a : fold_map(s, b, count, LOGF);
+    if (s.plain_rows) {
+        w.plain = plain_rows(s, a, b, 256 >> LOGF);
+    } else {
+        w.map_a = fold_map(s, poly_only == 1 ? b : a, count, LOGF);
+        w.map_b = poly_only == 0 ? w.map_a : fold_map(s, b, count, LOGF);
+    }
     w.work = work;
     w.ws_bstride = s.workspace_bytes / 4;
     w.n = int(s.n);
@@ -307,10 +326,10 @@ void launch_k1f(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
     w.count = int(count);
     w.log_groups = int(s.logC) - (LOGF + 3);
     const int items = int(count) * (poly_only < 0 ? 2 : 1) << w.log_groups;
-    auto kernel = k1f_convert<LOGF, PlanFoldWork>;
+    auto kernel = s.plain_rows ? k1f_convert<LOGF, PlanFoldWork, true> : k1f_convert<LOGF, PlanFoldWork>;
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k1f_smem_bytes())),
                "K1F shared memory");
-    kernel<<<std::min(items, s.sms), kFoldThreads, k1f_smem_bytes(), st>>>(
+    kernel<<<std::min(items, s.sms), k1f_threads(s.plain_rows), k1f_smem_bytes(), st>>>(
         w, s.basis->d_pc, s.basis->d_fold_weights + (LOGF - 1) * size_t(kFoldWeightBytes), s.basis->d_tw_fwd,
         int((s.qbits + 7) / 8), s.d_err);
 }
@@ -325,7 +344,7 @@ template <int LOGR>
 void launch_whole_basis(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
                         cudaStream_t st, int poly_only = -1) {
     const size_t tiles = size_t(count) * (poly_only < 0 ? 2 : 1) * s.n / tc::kTileM;
-    switch (LOGR == 4 && tiles > size_t(s.sms) * 4 ? plan_fold(s) : 0) {
+    switch (LOGR == 4 && tiles > size_t(s.sms) * 4 ? plan_fold(s, work) : 0) {
         case 1: return launch_k1f<1>(s, a, b, work, count, st, poly_only);
         case 2: return launch_k1f<2>(s, a, b, work, count, st, poly_only);
         case 3: return launch_k1f<3>(s, a, b, work, count, st, poly_only);
@@ -336,7 +355,7 @@ void launch_whole_basis(const PlanCore& s, const uint32_t* a, const uint32_t* b,
 template <int LOGR>
 void launch_conversion(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
                        cudaStream_t st) {
-    if (s.tune.conv_whole_basis)
+    if (s.tune.conv_whole_basis || s.plain_rows)  // (K1T loads by tensor maps only)
         launch_whole_basis<LOGR>(s, a, b, work, count, st);
     else
         launch_k1t<LOGR>(s, a, b, work, count, st);
@@ -359,7 +378,8 @@ void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t c
                "K3T shared memory");
     PlanCrtWork w;
     std::memset(&w.map_res, 0, sizeof w.map_res);
-    w.use_tma = (C * 4) % 16 == 0;  // rows of fewer than 4 columns cannot be described by a tensor map
+    // rows of fewer than 4 columns, or planes off a 16-byte boundary, cannot be described by a tensor map
+    w.use_tma = (C * 4) % 16 == 0 && reinterpret_cast<uintptr_t>(work) % 16 == 0;
     if (w.use_tma) w.map_res = residue_map(s, work, count, tc::kMaxPrimes);  // a constant row stride in the box
     w.work = work;
     w.out = c;
@@ -459,7 +479,7 @@ void launch_quartic(const PlanCore& s, const uint32_t* a, const uint32_t* b, uin
 }
 
 bool conversion_splits(const PlanCore& s) {
-    return (s.flags & PM_CONVERT_TENSOR) && !s.quartic && !s.wide && s.tune.conv_whole_basis;
+    return (s.flags & PM_CONVERT_TENSOR) && !s.quartic && !s.wide && (s.tune.conv_whole_basis || s.plain_rows);
 }
 
 void launch_tensor_convert_poly(const PlanCore& s, const uint32_t* x, int poly, uint32_t* work, cudaStream_t st) {

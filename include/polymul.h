@@ -40,9 +40,10 @@ enum pm_status {
 };
 
 /* Residue conversion and CRT implementation.  With neither PM_CONVERT_TENSOR nor
- * PM_CONVERT_SIMT a plan takes the tensor-core path whenever coef_limbs is even (16-byte
- * coefficient rows, which its tensor maps need; the FHERMA point's 14 limbs are), else
- * the plain method; pm_plan_info.convert says which one it runs. */
+ * PM_CONVERT_SIMT a plan takes the tensor-core path whenever coef_limbs is even or n >= 256
+ * (an odd coef_limbs has no 16-byte coefficient rows for tensor maps: its conversion loads
+ * rows without them), else the plain method; pm_plan_info.convert says which one it runs.
+ * PM_CONVERT_TENSOR asks for tensor maps and refuses an odd coef_limbs. */
 enum pm_flags {
     PM_CONVERT_DEFAULT = 0, /* the tensor path where the plan allows it, else the plain method */
     PM_CONVERT_TENSOR = 1,  /* exact INT8 digit contractions on the tcgen05 tensor cores */
@@ -129,7 +130,7 @@ int pm_plan_destroy(pm_plan* plan);
  * calls on one plan must not overlap).  Replaces the device half of fherma_run
  * (rns/solve.cu:504-578, launch_rns).
  * Pointers must be device, managed or pinned memory, 8-byte aligned; on the
- * tensor path a, b and workspace 16-byte aligned (cudaMalloc gives 256):
+ * tensor path with an even coef_limbs a, b and workspace 16-byte aligned (cudaMalloc gives 256):
  * otherwise PM_ERR_INVALID, before anything runs.  The call runs on the
  * current device, which must be the one the plan was created on, and device
  * pointers must be that device's memory: otherwise PM_ERR_INVALID too.  The
