@@ -22,6 +22,7 @@
 // Pinned caller buffers skip the staging: their pieces are copied directly.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -29,6 +30,7 @@
 #include <cstring>
 #include <functional>
 #include <immintrin.h>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -106,9 +108,44 @@ static long spin_us() {
     return us;
 }
 
-// Persistent host threads that run the pieces of one job; the calling thread
-// takes pieces too.  Idle workers spin for a short while (back-to-back calls
-// find them awake), then sleep on a condition variable.
+// One host copy in pieces: f(k) for k in [0, pieces), handed out in order, of which the first
+// `available` may run yet.
+struct CopyJob {
+    CopyJob(int n, const std::function<void(int)>& fn) : pieces(n), f(fn) {}
+    const int pieces;
+    const std::function<void(int)>& f;
+    std::atomic<int> available{0}, next{0}, done{0}, inside{0};
+    std::mutex error_m;
+    std::exception_ptr error;
+
+    // runs one available piece; false when none is left to take now
+    bool step() {
+        int k = next.load(std::memory_order_relaxed);
+        do {
+            if (k >= available.load(std::memory_order_acquire)) return false;
+        } while (!next.compare_exchange_weak(k, k + 1, std::memory_order_relaxed));
+        try {
+            f(k);
+        } catch (...) {
+            std::lock_guard<std::mutex> lock(error_m);
+            if (!error) error = std::current_exception();
+        }
+        done.fetch_add(1, std::memory_order_release);
+        return true;
+    }
+    bool left() const {
+        return next.load(std::memory_order_relaxed) < available.load(std::memory_order_acquire);
+    }
+};
+
+// Host threads that run the pieces of open copy jobs; each job's calling thread takes pieces
+// too.  Idle workers spin for a while (back-to-back calls find them awake), then sleep on
+// a condition variable.  Every plan of the process shares one pool, made with the first
+// plan that needs it and ended with the last: a pool per plan left each plan's threads
+// spinning through the other plans' calls (three plans called in turn on a 16-vCPU host took
+// 1010 us a call at N = 32768 against 350 alone; 345 with the shared pool).  Jobs of calls on several
+// threads are open side by side; workers never wait inside a piece, so one call's
+// pending pieces do not hold up another's.
 class CopyPool {
 public:
     explicit CopyPool(int threads) {
@@ -118,91 +155,67 @@ public:
         {
             std::lock_guard<std::mutex> lock(m_);
             stop_ = true;
-            ++generation_;
+            generation_.fetch_add(1, std::memory_order_release);
         }
         cv_.notify_all();
         for (auto& w : workers_) w.join();
     }
-    int threads() const { return int(workers_.size()); }
 
-    // Runs f(k) for k in [0, pieces) on the workers and the caller; returns when
-    // all are done and no worker is still inside the job.  The first exception a
-    // piece throws is rethrown here.
-    void run(int pieces, const std::function<void(int)>& f) {
+    // the process's pool, alive while any plan holds it
+    static std::shared_ptr<CopyPool> shared(int threads) {
+        static std::mutex m;
+        static std::weak_ptr<CopyPool> current;
+        std::lock_guard<std::mutex> lock(m);
+        std::shared_ptr<CopyPool> pool = current.lock();
+        if (!pool) {
+            pool = std::make_shared<CopyPool>(threads);
+            current = pool;
+        }
+        return pool;
+    }
+
+    void open(CopyJob& job, int available) {
         {
             std::lock_guard<std::mutex> lock(m_);
-            job_ = &f;
-            pieces_ = pieces;
-            next_.store(0);
-            done_.store(0);
-            error_ = nullptr;
+            job.available.store(available, std::memory_order_release);
+            jobs_.push_back(&job);
             generation_.fetch_add(1, std::memory_order_release);
         }
         cv_.notify_all();
-        work(&f, pieces);
-        while (done_.load(std::memory_order_acquire) < pieces) _mm_pause();
-        // no worker joins from here on (they join under the lock while job_ is set); the ones
-        // that joined find no piece left and leave before the next job resets the counters
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            job_ = nullptr;
-        }
-        while (active_.load(std::memory_order_acquire) > 0) _mm_pause();
-        if (error_) std::rethrow_exception(error_);
     }
-
-    // The same job without the caller: returns at once; finish() waits for it.
-    void start(int pieces, const std::function<void(int)>& f) {
+    // the job's first `available` pieces may run now
+    void publish(CopyJob& job, int available) {
         {
             std::lock_guard<std::mutex> lock(m_);
-            job_ = &f;
-            pieces_ = pieces;
-            next_.store(0);
-            done_.store(0);
-            error_ = nullptr;
+            job.available.store(available, std::memory_order_release);
             generation_.fetch_add(1, std::memory_order_release);
         }
         cv_.notify_all();
-        started_ = pieces;
-        job_started_ = &f;
     }
-    // The caller takes one piece of the started job, if one is left; false when none is.
-    bool help() {
-        const int pieces = started_;
-        const int k = next_.fetch_add(1);
-        if (k >= pieces) return false;
-        try {
-            (*job_started_)(k);
-        } catch (...) {
-            std::lock_guard<std::mutex> lock(m_);
-            if (!error_) error_ = std::current_exception();
-        }
-        done_.fetch_add(1, std::memory_order_release);
-        return true;
-    }
-    void finish() {
-        const int pieces = started_;
-        started_ = 0;
-        while (done_.load(std::memory_order_acquire) < pieces) _mm_pause();
+    // Ends the job: pieces already taken finish, the rest never start.  With `all`, waits for
+    // (and helps with) every piece first and rethrows the first exception a piece threw.
+    void close(CopyJob& job, bool all) {
+        if (all)
+            while (job.done.load(std::memory_order_acquire) < job.pieces)
+                if (!job.step()) _mm_pause();
         {
             std::lock_guard<std::mutex> lock(m_);
-            job_ = nullptr;
+            jobs_.erase(std::find(jobs_.begin(), jobs_.end(), &job));
         }
-        while (active_.load(std::memory_order_acquire) > 0) _mm_pause();
-        if (error_) std::rethrow_exception(error_);
+        job.next.store(job.pieces, std::memory_order_relaxed);
+        while (job.inside.load(std::memory_order_acquire) > 0) _mm_pause();
+        if (all && job.error) std::rethrow_exception(job.error);
     }
 
 private:
-    void work(const std::function<void(int)>* f, int pieces) {
-        for (int k = next_.fetch_add(1); k < pieces; k = next_.fetch_add(1)) {
-            try {
-                (*f)(k);
-            } catch (...) {
-                std::lock_guard<std::mutex> lock(m_);
-                if (!error_) error_ = std::current_exception();
+    // an open job with a piece to take, entered by the calling worker; null when there is none
+    CopyJob* enter() {
+        for (CopyJob* j : jobs_)
+            if (j->left()) {
+                j->inside.fetch_add(1, std::memory_order_acq_rel);
+                return j;
             }
-            done_.fetch_add(1, std::memory_order_release);
-        }
+        return nullptr;
     }
     void loop() {
         uint64_t seen = 0;
@@ -216,13 +229,13 @@ private:
             cv_.wait(lock, [&] { return generation_.load() != seen; });
             seen = generation_.load();
             if (stop_) return;
-            if (!job_) continue;  // that job is over already
-            const std::function<void(int)>* f = job_;
-            const int pieces = pieces_;
-            active_.fetch_add(1, std::memory_order_acq_rel);
-            lock.unlock();
-            work(f, pieces);
-            active_.fetch_sub(1, std::memory_order_acq_rel);
+            while (CopyJob* j = enter()) {
+                lock.unlock();
+                while (j->step()) {
+                }
+                j->inside.fetch_sub(1, std::memory_order_acq_rel);
+                lock.lock();
+            }
         }
     }
 
@@ -230,13 +243,8 @@ private:
     std::mutex m_;
     std::condition_variable cv_;
     std::atomic<uint64_t> generation_{0};
-    const std::function<void(int)>* job_ = nullptr;
-    int pieces_ = 0;
-    std::atomic<int> next_{0}, done_{0}, active_{0};
-    std::exception_ptr error_;
+    std::vector<CopyJob*> jobs_;
     bool stop_ = false;
-    int started_ = 0;
-    const std::function<void(int)>* job_started_ = nullptr;
 };
 
 namespace {
@@ -345,7 +353,7 @@ void multiply_host_begin(PlanCore& s, const uint64_t* a, const uint64_t* b, uint
         cuda_check(cudaEventCreateWithFlags(&h.a_in, cudaEventDisableTiming), "input event");
         cuda_check(cudaEventCreateWithFlags(&h.a_converted, cudaEventDisableTiming), "conversion event");
     }
-    if (!h.pool) h.pool = std::make_unique<CopyPool>(pool_threads());
+    if (!h.pool) h.pool = CopyPool::shared(pool_threads());
     const size_t io = s.io_bytes;
     uint8_t* dev = static_cast<uint8_t*>(h.d_io);
     uint8_t* stage = static_cast<uint8_t*>(h.h_stage);
@@ -384,13 +392,14 @@ void multiply_host_begin(PlanCore& s, const uint64_t* a, const uint64_t* b, uint
             if (len) host_copy(stage + poly * io + off, src[poly] + off, len);
             h.ready[k].store(1, std::memory_order_release);
         };
-        h.pool->start(nu, stage_unit);
+        CopyJob job(nu, stage_unit);
+        h.pool->open(job, nu);
         try {
             for (int grp = 0; grp < g.count; ++grp) {
                 // stage units too while this copy's are not all ready (the workers may be waking)
                 for (int k = grp * kGroupUnits; k < (grp + 1) * kGroupUnits; ++k)
                     while (!h.ready[k].load(std::memory_order_acquire))
-                        if (!h.pool->help()) _mm_pause();
+                        if (!job.step()) _mm_pause();
                 const size_t off = g.off[grp];
                 uint8_t* dst = dev + g.poly[grp] * io + off;
                 cuda_check(cudaMemcpyAsync(dst, stage + g.poly[grp] * io + off, g.len[grp], cudaMemcpyHostToDevice,
@@ -400,13 +409,10 @@ void multiply_host_begin(PlanCore& s, const uint64_t* a, const uint64_t* b, uint
                     convert_a_aside();
             }
         } catch (...) {
-            try {
-                h.pool->finish();
-            } catch (...) {
-            }
+            h.pool->close(job, false);
             throw;
         }
-        h.pool->finish();
+        h.pool->close(job, true);
     }
     if (a_aside) {
         launch_tensor_convert_poly(s, reinterpret_cast<const uint32_t*>(dev + io), 1, work, h.stream);
@@ -448,19 +454,16 @@ void multiply_host_end(PlanCore& s, uint64_t* c) {
         throw Failure(PM_ERR_INVALID, "the product was directed to another output buffer at the start of the call");
     // each product piece leaves the staging as soon as it has landed: this thread polls the
     // pieces' events in order (a blocking wait can sleep for longer than a piece takes) and
-    // flags them; the pool's threads copy the units of flagged pieces out
+    // hands their units to the pool's threads
     if (!h.direct_out) {
-        for (int k = 0; k < kOutPieces; ++k) h.ready[k].store(0, std::memory_order_relaxed);
         const std::function<void(int)> copy_unit = [&](int k) {  // unit k % 9 of piece k / 9
-            const int pc = k / kGroupUnits;
             size_t poff, plen, off, len;
-            out_piece(io, pc, &poff, &plen);
+            out_piece(io, k / kGroupUnits, &poff, &plen);
             piece(plen, kGroupUnits, k % kGroupUnits, &off, &len);
-            if (!len) return;
-            while (!h.ready[pc].load(std::memory_order_acquire)) _mm_pause();
-            host_copy(dst + poff + off, stage + 2 * io + poff + off, len);
+            if (len) host_copy(dst + poff + off, stage + 2 * io + poff + off, len);
         };
-        h.pool->start(kOutPieces * kGroupUnits, copy_unit);
+        CopyJob job(kOutPieces * kGroupUnits, copy_unit);
+        h.pool->open(job, 0);
         try {
             const auto give_up = std::chrono::steady_clock::now() + std::chrono::seconds(60);
             for (int k = 0; k < kOutPieces; ++k) {
@@ -471,19 +474,13 @@ void multiply_host_end(PlanCore& s, uint64_t* c) {
                     _mm_pause();
                 }
                 cuda_check(e, "product");
-                h.ready[k].store(1, std::memory_order_release);
+                h.pool->publish(job, (k + 1) * kGroupUnits);
             }
         } catch (...) {
-            for (int k = 0; k < kOutPieces; ++k) h.ready[k].store(1, std::memory_order_release);  // release the copiers
-            try {
-                h.pool->finish();
-            } catch (...) {
-            }
+            h.pool->close(job, false);
             throw;
         }
-        while (h.pool->help()) {
-        }
-        h.pool->finish();
+        h.pool->close(job, true);
     }
     cuda_check(cudaStreamSynchronize(h.stream), "product");
     uint32_t herr = 0;

@@ -79,7 +79,7 @@ struct HostCall {
     void* d_io = nullptr;           // a, b, c on the device
     void* h_stage = nullptr;        // pinned a, b, c and the error word
     std::vector<cudaEvent_t> out_ready;
-    std::unique_ptr<CopyPool> pool;
+    std::shared_ptr<CopyPool> pool;  // the process's copy threads
     std::atomic<uint8_t> ready[64];  // input piece k staged
     bool pending = false;           // between multiply_host_begin and multiply_host_end
     uint8_t* direct_out = nullptr;  // pinned caller output the product lands in directly, or null
