@@ -88,6 +88,8 @@ struct HostCall {
 
 // Largest launch group by default, and the largest a caller may set.
 constexpr uint32_t kMaxDefaultGroup = 128;
+constexpr size_t kSmallGroupBytes = size_t(64) << 20;  // residue planes up to which a default group may pass that,
+constexpr uint32_t kMaxSmallGroup = 4096;              // up to this many products (grid dimensions)
 constexpr uint32_t kMaxGroup = 256;
 
 // Launch shapes the autotuner chooses per plan (defaults apply until it runs).

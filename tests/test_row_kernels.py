@@ -46,3 +46,25 @@ def test_row_lengths_and_radices(cuda, n, tensor):
             torch.cuda.synchronize()
             assert (c.cpu().numpy().view(np.uint64) == want).all(), (radix, persistent)
             assert (one.cpu().numpy().view(np.uint64) == want[0]).all(), (radix, persistent)
+
+
+@pytest.mark.parametrize("tensor", [True, False])
+@pytest.mark.parametrize("n,count", [(2, 4099), (16, 4099), (256, 1500)])
+def test_large_default_groups_of_small_products(cuda, n, count, tensor):
+    """More products than one default group of small rings holds: the same bits as groups of 100."""
+    torch = cuda
+    q = random_q(np.random.default_rng(n + count), 90)
+    rng = np.random.default_rng(count)
+    a, b = (uniform_below(rng, q, n * count, 2).reshape(count, n, 2) for _ in range(2))
+    da, db = (torch.from_numpy(x.view(np.int64)).cuda() for x in (a, b))
+    with polymul.Plan(n, q, 2, tensor=tensor) as p:
+        outs = []
+        for group in (0, 100):
+            p.set_tuning(group=group)
+            c = torch.zeros_like(da)
+            p.multiply_batch(da.data_ptr(), db.data_ptr(), c.data_ptr(), count)
+            torch.cuda.synchronize()
+            outs.append(c)
+        assert torch.equal(outs[0], outs[1])
+    for k in (0, 128, 4096 if count > 4096 else 1300, count - 1):
+        assert (outs[0][k].cpu().numpy().view(np.uint64) == oracle.rns_multiply(a[k], b[k], q)).all()
