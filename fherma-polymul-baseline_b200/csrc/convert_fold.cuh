@@ -184,6 +184,10 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
                 tc::mbar_expect_tx(&w_full, kFoldWeightBytes);
                 for (uint32_t o = 0; o < kFoldWeightBytes; o += 32768) tc::bulk_load(sW + o, weights + o, 32768u, &w_full);
             }
+        }
+        grid_trigger();
+        grid_wait();  // the coefficients, and the planes' previous readers; the epilogue only follows the MMAs
+        if (tiles > 0) {
             if (!PLAIN)
                 for (; issued < kFoldTiles && issued < tiles; ++issued)
                     if (lane == 0) issue(issued);
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
                 tc::mbar_arrive(&tma_full[kk % kFoldTiles]);
             };
             int loaded = 0;
+            grid_wait();  // the coefficients
             for (int kk = 0; kk < tiles; ++kk, ++loaded) {
                 const int b = kk % kFoldTiles;
                 if (kk >= kFoldTiles)  // the MMAs have read the buffer's last tile

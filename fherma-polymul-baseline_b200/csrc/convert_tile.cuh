@@ -174,6 +174,8 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
             tc::mbar_expect_tx(&b_full, 32768u);
             tc::bulk_load(sB, conv_w, 32768u, &b_full);
         }
+        grid_trigger();
+        grid_wait();  // the coefficients, and the planes' previous readers; the workers only follow this warp
         if ((PLAIN || lane == 0) && begin < end) {
             issue(begin, 0);
             if (begin + 1 < end) issue(begin + 1, 1);

@@ -58,6 +58,25 @@ void twiddle_tables(uint32_t p, uint2* fwd, uint2* inv);
 std::vector<uint32_t> make_primes();
 unsigned basis_size(const std::vector<uint32_t>& primes, unsigned n, unsigned qbits);
 
+// Launch as a programmatic dependent of the stream's previous kernel (only kernels that call
+// grid_wait before they touch what earlier kernels write or read).  early = false: a plain launch,
+// where the kernel also depends on another stream's event.
+template <class... Params, class... Args>
+void launch_dependent(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    cuda_check(cudaLaunchKernelEx(&cfg, kernel, Params(args)...), "launch");
+}
+
 // One stage of the host-batch pipeline: a stream with its own device buffers
 // (a, b, c and the residue workspace of a group) and pinned staging.
 struct PipelineSlot {
@@ -188,7 +207,7 @@ struct PlanCore {
 void launch_simt(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_t* work,
                  uint32_t count, cudaStream_t st);
 uint32_t group_size(const PlanCore& s);
-void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t st);
+void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t st, bool early = true);
 void check_device_errors(const PlanCore& s);
 // Device-pointer arguments a kernel may touch: reachable from the device (not
 // pageable host memory), 8-byte aligned (u64 coefficients; the kernels move 8

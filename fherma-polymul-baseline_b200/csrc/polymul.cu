@@ -433,6 +433,7 @@ struct Batch {
     uint32_t count;     // products in this launch
     size_t io_bstride;  // words between consecutive products' a (b, c)
     size_t ws_bstride;  // words between consecutive products' residue planes
+    bool early = true;  // the row kernel may start as a programmatic dependent
 };
 
 template <int W>
@@ -473,8 +474,8 @@ void launch_k2_fixed(const PlanCore& s, uint32_t* work, const Batch& bt, cudaStr
             const size_t smem = k2w_smem_bytes<LOGC>();
             const PlanWarpRowWork w{work, bt.ws_bstride, int(s.n), int(s.logR), int(s.logC), int(s.P), int(bt.count)};
             const int64_t items = int64_t(s.P) * ((1 << s.logR) / warp_rows(LOGC, int(s.logR))) * bt.count;
-            k2w_rows<LOGC, PlanWarpRowWork><<<k2w_grid(items, s.sms), 32 * kWarpRowWarps, smem, st>>>(
-                w, s.plane_pc(), s.plane_fwd(), s.plane_inv(), int(s.logR));
+            launch_dependent(bt.early, k2w_rows<LOGC, PlanWarpRowWork>, k2w_grid(items, s.sms), 32 * kWarpRowWarps, smem, st, w,
+                             s.plane_pc(), s.plane_fwd(), s.plane_inv(), int(s.logR));
             return;
         }
     }
@@ -489,8 +490,8 @@ void launch_k2_fixed(const PlanCore& s, uint32_t* work, const Batch& bt, cudaStr
             const int64_t total = items * bt.count;
             const int ctas = int(std::min<int64_t>(total, int64_t(s.sms) * k2p_min_blocks(LOGC)));
             const PlanRowWork w{work, bt.ws_bstride, int(s.n), int(s.logR), int(s.logC), int(s.P), int(bt.count)};
-            k2p_rows<LOGC, KP, PlanRowWork><<<ctas, k2p_threads(LOGC, KP), smem, st>>>(
-                w, s.plane_pc(), s.plane_fwd(), s.plane_inv(), int(s.logR), s.d_err);
+            launch_dependent(bt.early, k2p_rows<LOGC, KP, PlanRowWork>, ctas, k2p_threads(LOGC, KP), smem, st, w, s.plane_pc(),
+                             s.plane_fwd(), s.plane_inv(), int(s.logR), s.d_err);
             return;
         }
     }
@@ -554,8 +555,8 @@ void launch_k2(const PlanCore& s, uint32_t* work, const Batch& bt, cudaStream_t 
     }
 }  // namespace
 
-void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t st) {
-    launch_k2(s, work, Batch{count, size_t(s.n) * s.stride, s.workspace_bytes / 4}, st);
+void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t st, bool early) {
+    launch_k2(s, work, Batch{count, size_t(s.n) * s.stride, s.workspace_bytes / 4, early}, st);
 }
 
 void launch_simt(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_t* work,

@@ -86,6 +86,8 @@ __global__ void __launch_bounds__(k2p_threads(LOGC, KP), k2p_min_blocks(LOGC))
     }
     tc::fence_smem_async();
     __syncthreads();
+    grid_trigger();
+    grid_wait();  // the conversion's planes
 
     auto issue_rows = [&](int k) {
         const RowItem it = w.item(k);

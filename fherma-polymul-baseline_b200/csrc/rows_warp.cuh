@@ -249,6 +249,26 @@ __global__ void __launch_bounds__(32 * kWarpRowWarps, 5)
     const bool live = slot < rows;  // (planes of fewer than 512 values leave lanes idle)
     int cur_i = -1, cur_r = -1;
     PrimeConst pc{};
+    // the rows' twiddles: row slot's entry j = 2^s + i' is Psi_rev[(R + r) 2^s + i'], s < log2 C - 2
+    auto stage_twiddles = [&](const RowItem& it) {
+        const uint2* gf = tw_fwd + size_t(it.i) * kNMax;
+        const uint2* gi = tw_inv + size_t(it.i) * kNMax;
+        for (int e = lane; e < rows * (W::C / 4); e += 32) {
+            const int sl = e / (W::C / 4), j = e & (W::C / 4 - 1);
+            if (j == 0) continue;
+            const int s = 31 - __clz(j);
+            const int g = ((R + it.r + sl) << s) + (j - (1 << s));
+            stf[sl * W::TWS + j] = __ldg(gf + g);
+            sti[sl * W::TWS + j] = __ldg(gi + g);
+        }
+        pc = pcs[it.i];
+        cur_i = it.i;
+        cur_r = it.r;
+        __syncwarp();
+    };
+    grid_trigger();
+    if (begin < end) stage_twiddles(w.item(begin));
+    grid_wait();  // the conversion's planes
     for (int k = begin; k < end; ++k) {
         const RowItem it = w.item(k);
         uint32_t* ga = it.a + slot * W::C + t * W::G;
@@ -266,21 +286,7 @@ __global__ void __launch_bounds__(32 * kWarpRowWarps, 5)
         }
         if (it.i != cur_i || it.r != cur_r) {
             __syncwarp();  // every lane is done with the previous rows' twiddles
-            // row slot's entry j = 2^s + i' is Psi_rev[(R + r) 2^s + i'], s < log2 C - 2
-            const uint2* gf = tw_fwd + size_t(it.i) * kNMax;
-            const uint2* gi = tw_inv + size_t(it.i) * kNMax;
-            for (int e = lane; e < rows * (W::C / 4); e += 32) {
-                const int sl = e / (W::C / 4), j = e & (W::C / 4 - 1);
-                if (j == 0) continue;
-                const int s = 31 - __clz(j);
-                const int g = ((R + it.r + sl) << s) + (j - (1 << s));
-                stf[sl * W::TWS + j] = __ldg(gf + g);
-                sti[sl * W::TWS + j] = __ldg(gi + g);
-            }
-            pc = pcs[it.i];
-            cur_i = it.i;
-            cur_r = it.r;
-            __syncwarp();
+            stage_twiddles(it);
         }
         const int ts = live ? slot : 0;
         warp_row_product<LOGC>(va, vb, sa, sb, stf + ts * W::TWS, sti + ts * W::TWS, lane, pc);

@@ -285,7 +285,8 @@ void launch_k1w(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
             fix.shift[t] = s.quartic->fix_shift[t];
         }
     }
-    kernel<<<ctas, tc::kWideThreads, smem, st>>>(w, s.plane_pc(), s.conv_weights(), s.plane_fwd(), s.d_err, fix);
+    launch_dependent(poly_only < 0, kernel, ctas, tc::kWideThreads, smem, st, w, s.plane_pc(), s.conv_weights(), s.plane_fwd(), s.d_err,
+                     fix);
 }
 
 // Coefficient bytes for K1F: boxes of the row block's (256 >> f) bytes x 2^(f + 3) columns x 16 >> f rows.
@@ -329,9 +330,9 @@ void launch_k1f(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
     auto kernel = s.plain_rows ? k1f_convert<LOGF, PlanFoldWork, true> : k1f_convert<LOGF, PlanFoldWork>;
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k1f_smem_bytes())),
                "K1F shared memory");
-    kernel<<<std::min(items, s.sms), k1f_threads(s.plain_rows), k1f_smem_bytes(), st>>>(
-        w, s.basis->d_pc, s.basis->d_fold_weights + (LOGF - 1) * size_t(kFoldWeightBytes), s.basis->d_tw_fwd,
-        int((s.qbits + 7) / 8), s.d_err);
+    launch_dependent(poly_only < 0, kernel, std::min(items, s.sms), k1f_threads(s.plain_rows), k1f_smem_bytes(), st, w, s.basis->d_pc,
+                     s.basis->d_fold_weights + (LOGF - 1) * size_t(kFoldWeightBytes), s.basis->d_tw_fwd,
+                     int((s.qbits + 7) / 8), s.d_err);
 }
 
 // Conversion of both polynomials (poly_only < 0) or of one, by the folding kernel or K1W.  K1F
@@ -398,7 +399,7 @@ void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t c
     w.P = int(s.P);
     w.stride = int(s.stride);
     w.count = int(count);
-    kernel<<<ctas, tc::kCrtThreads, smem, st>>>(w, s.plane_pc(), s.plane_inv(), s.d_err);
+    launch_dependent(true, kernel, ctas, tc::kCrtThreads, smem, st, w, s.plane_pc(), s.plane_inv(), s.d_err);
 }
 
 template <int LOGR>
@@ -502,7 +503,7 @@ void launch_tensor_after_conversion(const PlanCore& s, uint32_t* c, uint32_t* wo
                                     cudaStream_t st) {
     {
         ProfileScope prof("k2_rows", st);
-        launch_rows(s, work, count, st);
+        launch_rows(s, work, count, st, false);  // both polynomials' conversions, on two streams
     }
     {
         ProfileScope prof("k3t_cols_crt", st);

@@ -498,12 +498,12 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
         tc::mbar_expect_tx(&tma_bar, uint32_t(tc::kMaxPrimes * R * Gc) * 4u);  // the whole box, absent primes zero-filled
         tc::tma_load_4d(sR, t.map, it.y * Gc, 0, 0, t.mz, &tma_bar);
     };
-    if (tid == 0 && begin < end) issue(begin);
-
     const uint8_t* cur_w = nullptr;  // the product whose tables are in shared memory
     int cur_P = 0;
     uint32_t tma_phase = 0, mma_phase = 0;
     bool ok = true;
+    grid_trigger();
+    if (begin >= end) grid_wait();
     for (int k = begin; k < end; ++k) {
         const int2 it = w.item(k);
         const CrtTarget t = w.target(it.x);
@@ -529,6 +529,10 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
             cur_P = t.P;
             tc::fence_smem_async();
             __syncthreads();
+        }
+        if (k == begin) {
+            grid_wait();  // the row kernel's planes, and the output's previous readers
+            if (tid == 0) issue(k);
         }
         if (t.use_tma) {
             ok = tc::mbar_wait(&tma_bar, tma_phase) && ok;
