@@ -4,8 +4,10 @@
 // (prime basis sized for its N and bits(q), CRT constants and weights),
 // packed device buffers for a, b, c and the residue planes, per-product tensor
 // maps, and flat work tables:
-//   conversion items  (product, prime group, polynomial, column group) ordered
-//                     prime group first -- one persistent launch of k1t_convert;
+//   conversion items  (product, polynomial, column group) per number of folded
+//                     column stages (three, two or one, by the product's basis) --
+//                     one persistent launch of k1f_convert per class, each on its
+//                     share of the SMs;
 //   row items         (product, prime, first row) per ring size class -- one
 //                     launch per class: the persistent k2p_rows for rows of
 //                     1024 values or more (items prime/row first, so a CTA
@@ -29,9 +31,29 @@
 #include "pm_internal.h"
 #include "rows_persistent.cuh"
 #include "rows_warp.cuh"
+#include "convert_fold.cuh"
 #include "tensor_kernels.cuh"
 
 namespace pm {
+
+// conversion tiles of one class from a table of (product, polynomial, column group) items
+struct TableFoldWork {
+    const uint4* items;
+    int nitems;
+    const BatchProduct* prod;
+    const CUtensorMap* maps;  // [3 * products]: a, b, residues
+    uint32_t* work;
+    PlainRows plain;  // (not used: batches have 16-byte coefficient rows)
+    __device__ int total() const { return nitems; }
+    __device__ TileItem item(int k) const {
+        const uint4 v = items[k];
+        return TileItem{int(v.x), int(v.y), int(v.z)};
+    }
+    __device__ ConvTarget target(int z, int poly) const {
+        const BatchProduct& d = prod[z];
+        return ConvTarget{maps + 3 * z + poly, 0, work + d.ws_off, d.n, d.logC, d.P};
+    }
+};
 
 // rows of one size class from a table of (product, prime, first row) items
 struct TableRowWork {
@@ -79,6 +101,16 @@ CUtensorMap encode(CUtensorMapDataType type, const void* base, const cuuint64_t 
                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw Failure(PM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a batch product");
     return map;
+}
+
+template <int LOGF>
+void launch_fold_class(const TableFoldWork& w, int ctas, int qbytes, const DeviceBasis& B, uint32_t* err,
+                       cudaStream_t st) {
+    cuda_check(cudaFuncSetAttribute(k1f_convert<LOGF, TableFoldWork>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(k1f_smem_bytes())),
+               "batch conversion shared memory");
+    k1f_convert<LOGF, TableFoldWork><<<ctas, k1f_threads(false), k1f_smem_bytes(), st>>>(
+        w, B.d_pc, B.d_fold_weights + (LOGF - 1) * size_t(kFoldWeightBytes), B.d_tw_fwd, qbytes, err);
 }
 
 template <int LOGC, int KP>
@@ -169,7 +201,11 @@ struct BatchCore {
     uint4* d_row_items = nullptr;
     uint2* d_crt_items = nullptr;
     uint32_t* d_err = nullptr;
-    int conv_items = 0;
+    struct FoldClass {
+        int f, count, ctas, qbytes;
+        size_t offset;  // into d_conv_items
+    };
+    std::vector<FoldClass> fold_classes;
     struct RowClass {
         int logC, radix_log, count;
         size_t offset;  // into d_row_items
@@ -183,7 +219,7 @@ struct BatchCore {
     cudaGraphExec_t graph = nullptr;
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> events;
-    int conv_ctas_per_sm = 3, crt_ctas_per_sm = 2;  // persistent grid sizes (autotuned)
+    int crt_ctas_per_sm = 2;  // persistent grid size (autotuned)
 
     ~BatchCore() {
         cudaSetDevice(device);
@@ -206,10 +242,6 @@ struct BatchCore {
     void enqueue(cudaStream_t st0) {
         const DeviceBasis& B = *plans[0]->basis;
         const int sms = sm_count_dev();
-        TableConvWork cw{d_conv_items, conv_items, d_prod, d_maps, d_work};
-        k1t_convert<4, TableConvWork><<<std::min(conv_items, sms * conv_ctas_per_sm), tc::kConvThreads, k1t_smem_bytes(), st0>>>(
-            cw, B.d_pc, B.d_conv_weights, B.d_tw_fwd, d_err);
-        cuda_check(cudaGetLastError(), "batch conversion launch");
         auto fork = [&](size_t k) {
             cudaStream_t s = streams[1 + k % (streams.size() - 1)];
             cuda_check(cudaEventRecord(events[0], st0), "batch fork");
@@ -222,6 +254,20 @@ struct BatchCore {
             cuda_check(cudaStreamWaitEvent(st0, e, 0), "batch join");
         };
         std::vector<cudaStream_t> used;
+        for (size_t k = 0; k < fold_classes.size(); ++k) {
+            const FoldClass& fc = fold_classes[k];
+            cudaStream_t s = fork(k);
+            const TableFoldWork w{d_conv_items + fc.offset, fc.count, d_prod, d_maps, d_work, PlainRows{}};
+            switch (fc.f) {
+                case 1: launch_fold_class<1>(w, fc.ctas, fc.qbytes, B, d_err, s); break;
+                case 2: launch_fold_class<2>(w, fc.ctas, fc.qbytes, B, d_err, s); break;
+                default: launch_fold_class<3>(w, fc.ctas, fc.qbytes, B, d_err, s); break;
+            }
+            used.push_back(s);
+        }
+        cuda_check(cudaGetLastError(), "batch conversion launch");
+        for (size_t k = 0; k < used.size(); ++k) join(used[k], k);
+        used.clear();
         for (size_t k = 0; k < row_classes.size(); ++k) {
             const RowClass& rc = row_classes[k];
             cudaStream_t s = fork(k);
@@ -290,13 +336,14 @@ struct BatchCore {
             const PlanCore& p = *plans[z];
             const cuuint64_t C = 1ull << p.logC, R = 1ull << p.logR, sb = p.stride * 4ull;
             const cuuint32_t Gc = cuuint32_t(C < 8 ? C : 8);
+            const int f = fold_stages(int(p.P), int(p.logC));  // at least one: n >= 256
             const cuuint64_t cdims[4] = {sb, C, R, 1};
             const cuuint64_t cstr[3] = {sb, sb * C, sb * C * R};
-            const cuuint32_t cbox[4] = {128, Gc, cuuint32_t(R), 1};
-            maps[3 * z] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_a + io_off[z], cdims, cstr, cbox,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
-            maps[3 * z + 1] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_b + io_off[z], cdims, cstr, cbox,
-                                     CU_TENSOR_MAP_SWIZZLE_128B);
+            const cuuint32_t cbox[4] = {256u >> f, 8u << f, 16u >> f, 1};
+            const CUtensorMapSwizzle swizzle =
+                f == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : (f == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+            maps[3 * z] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_a + io_off[z], cdims, cstr, cbox, swizzle);
+            maps[3 * z + 1] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_b + io_off[z], cdims, cstr, cbox, swizzle);
             // box lands as [row][64 primes][column]: a constant row stride (primes past P read as zero)
             const cuuint64_t rdims[4] = {C, p.P, R, 1};
             const cuuint64_t rstr[3] = {C * R * 4, C * 4, p.workspace_bytes};
@@ -305,16 +352,27 @@ struct BatchCore {
                                      CU_TENSOR_MAP_SWIZZLE_NONE);
         }
         // work tables
+        std::map<int, std::vector<uint4>> conv_by_f;
+        std::map<int, int> qbytes_by_f;
+        size_t tiles = 0;
+        for (uint32_t z = 0; z < cnt; ++z) {
+            const PlanCore& p = *plans[z];
+            const int f = fold_stages(int(p.P), int(p.logC));
+            const uint32_t groups = (1u << p.logC) / (8u << f);
+            for (uint32_t poly = 0; poly < 2; ++poly)
+                for (uint32_t cg = 0; cg < groups; ++cg) conv_by_f[f].push_back(make_uint4(z, poly, cg, 0));
+            qbytes_by_f[f] = std::max(qbytes_by_f[f], int((p.qbits + 7) / 8));
+            tiles += 2 * size_t(groups);
+        }
         std::vector<uint4> conv;
-        for (int pg = 0; pg < 4; ++pg)
-            for (uint32_t z = 0; z < cnt; ++z) {
-                const PlanCore& p = *plans[z];
-                if (pg * 16 >= int(p.P)) continue;
-                const uint32_t groups = (1u << p.logC) / 8;
-                for (uint32_t poly = 0; poly < 2; ++poly)
-                    for (uint32_t cg = 0; cg < groups; ++cg) conv.push_back(make_uint4(z, pg, poly, cg));
-            }
-        conv_items = int(conv.size());
+        const int sms = sm_count_dev();
+        for (auto& [f, items] : conv_by_f) {
+            // a CTA fills an SM: the classes run side by side on shares of them by their tiles
+            const int share = int(size_t(sms) * items.size() / tiles);
+            const int ctas = std::min(int(items.size()), std::max(1, share));
+            fold_classes.push_back(FoldClass{f, int(items.size()), ctas, qbytes_by_f[f], conv.size()});
+            conv.insert(conv.end(), items.begin(), items.end());
+        }
         std::map<int, std::vector<uint4>> rows_by_c;
         for (uint32_t z = 0; z < cnt; ++z) {
             const PlanCore& p = *plans[z];
@@ -357,7 +415,7 @@ struct BatchCore {
         upload(&d_row_items, row_items, "batch row items");
         upload(&d_crt_items, crt_items, "batch CRT items");
         // streams for capture: the main one and one per concurrent class
-        const size_t branches = std::max<size_t>(2, std::max(row_classes.size(), crt_classes.size()) + 1);
+        const size_t branches = std::max<size_t>(2, std::max(fold_classes.size(), std::max(row_classes.size(), crt_classes.size())) + 1);
         streams.resize(branches);
         events.resize(branches);
         for (auto& s : streams) cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "batch stream");
@@ -372,9 +430,6 @@ struct BatchCore {
             cudaGraphExecDestroy(graph);
             graph = nullptr;
         }
-        cuda_check(cudaFuncSetAttribute(k1t_convert<4, TableConvWork>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(k1t_smem_bytes())),
-                   "batch conversion shared memory");
         enqueue(streams[0]);
         cuda_check(cudaStreamSynchronize(streams[0]), "batch warm-up");
         cudaGraph_t g = nullptr;
@@ -429,11 +484,6 @@ struct BatchCore {
                 if (k == cur || rc.logC < 10) continue;  // the warp kernel's passes are fixed
                 attempt([&] { rc.radix_log = k; }, [&] { rc.radix_log = cur; });
             }
-        for (int k : {2, 3, 4}) {
-            const int old = conv_ctas_per_sm;
-            if (k == old) continue;
-            attempt([&] { conv_ctas_per_sm = k; }, [&] { conv_ctas_per_sm = old; });
-        }
         {
             const int old = crt_ctas_per_sm;
             attempt([&] { crt_ctas_per_sm = 1; }, [&] { crt_ctas_per_sm = old; });

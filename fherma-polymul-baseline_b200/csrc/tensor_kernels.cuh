@@ -5,7 +5,7 @@
 // each one is and where its product's data lives:
 //   PlanConvWork / PlanCrtWork   `count` products of one plan, items computed
 //                                from the index (maps are kernel parameters);
-//   TableConvWork / TableCrtWork products of different n and q (an uneven
+//   TableCrtWork                 products of different n and q (an uneven
 //                                batch), items and per-product descriptors read
 //                                from device tables (maps in global memory).
 // Each CTA takes a contiguous chunk of items, so the operand tables it keeps in
@@ -113,27 +113,6 @@ struct PlanConvWork {
         if (pg >= pgs) return make_int2(0, 0);
         const int chunk = (per_pg + m - 1) / m;
         return make_int2(pg * per_pg + min(j * chunk, per_pg), pg * per_pg + min((j + 1) * chunk, per_pg));
-    }
-};
-
-struct TableConvWork {
-    const uint4* items;  // (z, pg, poly, cg)
-    int nitems;
-    const BatchProduct* prod;
-    const CUtensorMap* maps;  // [3 * products]: a, b, residues
-    uint32_t* work;
-    __device__ int total() const { return nitems; }
-    __device__ ConvItem item(int k) const {
-        const uint4 v = items[k];
-        return ConvItem{int(v.x), int(v.y), int(v.z), int(v.w)};
-    }
-    __device__ ConvTarget target(int z, int poly) const {
-        const BatchProduct& d = prod[z];
-        return ConvTarget{maps + 3 * z + poly, 0, work + d.ws_off, d.n, d.logC, d.P};
-    }
-    __device__ int2 range(int b, int grid) const {  // contiguous runs of the table
-        const int chunk = (nitems + grid - 1) / grid;
-        return make_int2(min(nitems, b * chunk), min(nitems, (b + 1) * chunk));
     }
 };
 
