@@ -163,7 +163,7 @@ void launch_rows_any(int logC, int radix_log, const uint4* items, int count, con
 
 template <int W>
 void launch_crt_class(const TableCrtWork& w, int ctas, const DeviceBasis& B, uint32_t* err, cudaStream_t st) {
-    const size_t smem = k3t_smem_bytes<4>();
+    const size_t smem = k3t_smem_bytes<4>(W);
     cuda_check(cudaFuncSetAttribute(k3t_crt<4, W, TableCrtWork>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     int(smem)),
                "batch CRT shared memory");
@@ -281,7 +281,7 @@ struct BatchCore {
             const CrtClass& cc = crt_classes[k];
             cudaStream_t s = fork(k);
             TableCrtWork w{d_crt_items + cc.offset, cc.count, d_prod, d_maps, d_work, reinterpret_cast<uint32_t*>(d_c)};
-            launch_crt_any(cc.W, w, std::min(cc.count, sms * crt_ctas_per_sm), B, d_err, s);
+            launch_crt_any(cc.W, w, std::min(cc.count, sms * k3t_ctas_per_sm(cc.W, crt_ctas_per_sm)), B, d_err, s);
             used.push_back(s);
         }
         for (size_t k = 0; k < used.size(); ++k) join(used[k], k);
@@ -344,10 +344,10 @@ struct BatchCore {
                 f == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : (f == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
             maps[3 * z] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_a + io_off[z], cdims, cstr, cbox, swizzle);
             maps[3 * z + 1] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_b + io_off[z], cdims, cstr, cbox, swizzle);
-            // box lands as [row][64 primes][column]: a constant row stride (primes past P read as zero)
+            // box lands as [row][32 or 64 primes][column]: a constant row stride (primes past P read as zero)
             const cuuint64_t rdims[4] = {C, p.P, R, 1};
             const cuuint64_t rstr[3] = {C * R * 4, C * 4, p.workspace_bytes};
-            const cuuint32_t rbox[4] = {Gc, cuuint32_t(tc::kMaxPrimes), cuuint32_t(R), 1};
+            const cuuint32_t rbox[4] = {Gc, cuuint32_t(crt_cap(int(p.W))), cuuint32_t(R), 1};
             maps[3 * z + 2] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT32, d_work + ws_off[z], rdims, rstr, rbox,
                                      CU_TENSOR_MAP_SWIZZLE_NONE);
         }

@@ -366,9 +366,9 @@ template <int LOGR, int W>
 void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t count, cudaStream_t st) {
     const int C = 1 << s.logC, Gc = C < 8 ? C : 8;
     const int items = int(count) * (C / Gc);
-    int ctas = s.sms * s.tune.crt_ctas_per_sm;
+    int ctas = s.sms * k3t_ctas_per_sm(W, s.tune.crt_ctas_per_sm);
     if (ctas > items) ctas = items;
-    const size_t smem = k3t_smem_bytes<LOGR>();
+    const size_t smem = k3t_smem_bytes<LOGR>(W);
     // the reduction mod q is a table row: the same kernel for a special-form q; rows of 1024,
     // 2048 or 4096 values (n = 16384 .. 65536) take a kernel with that row length built in
     auto kernel = k3t_crt<LOGR, W, PlanCrtWork>;
@@ -381,7 +381,7 @@ void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t c
     std::memset(&w.map_res, 0, sizeof w.map_res);
     // rows of fewer than 4 columns, or planes off a 16-byte boundary, cannot be described by a tensor map
     w.use_tma = (C * 4) % 16 == 0 && reinterpret_cast<uintptr_t>(work) % 16 == 0;
-    if (w.use_tma) w.map_res = residue_map(s, work, count, tc::kMaxPrimes);  // a constant row stride in the box
+    if (w.use_tma) w.map_res = residue_map(s, work, count, uint32_t(crt_cap(W)));  // a constant row stride in the box
     w.work = work;
     w.out = c;
     w.ws_bstride = s.workspace_bytes / 4;

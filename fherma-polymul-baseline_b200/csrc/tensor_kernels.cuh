@@ -425,24 +425,34 @@ __device__ __forceinline__ void add1_carry(uint32_t& a, uint32_t b, uint32_t& cy
 // then also hit 32 distinct banks of the 128-byte swizzle.
 // The CRT weights, q constants and column twiddles of the current product stay
 // in shared memory until an item of another product needs its own.
-// Dynamic shared memory (1024-aligned): A 2 x 16 KB (K = 256), B 2 x 16 KB,
-// residue box 64*R*8 words, inverse column twiddles 64*(R-1) uint2.
+// Dynamic shared memory (1024-aligned), for crt_cap(W) = 64 primes (32: half of each): A 2 x 16 KB
+// (K = 256), B 2 x 16 KB, residue box 64*R*8 words, inverse column twiddles 64*(R-1) uint2.
 // ---------------------------------------------------------------------------
+// Primes a tile holds: W <= 12 words (q of up to 384 bits) need at most 27, so those kernels take
+// boxes, digit tiles and weights of 32 instead of 64 (52 KB a CTA instead of 104) and only the K
+// steps the primes fill; three CTAs share an SM.  Measured for 500 products of 200 bits at n = 1024:
+// 37.2 -> 31.3 us; an uneven batch of 200 to 868 bits, whole, 401 -> 390.
+constexpr int crt_cap(int W) { return W <= 12 ? 32 : 64; }
+constexpr int k3t_min_blocks(int W) { return W <= 12 ? 3 : 2; }
+// CTAs per SM of a launch: the tuning's default of two stands for as many as fit
+constexpr int k3t_ctas_per_sm(int W, int tuned) { return tuned == 2 ? k3t_min_blocks(W) : tuned; }
+
 // LOGC > 0: every item's rows hold 2^LOGC values (a plan's launch at a common ring size), so
 // the tile's column count and the output offsets are constants; 0: read from the item.
 template <int LOGR, int W, class Work, int LOGC = 0>
-__global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_constant__ Work w, const PrimeConst* __restrict__ pcs,
+__global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(const __grid_constant__ Work w, const PrimeConst* __restrict__ pcs,
                                                const uint2* __restrict__ tw_inv, uint32_t* __restrict__ err) {
     constexpr int R = 1 << LOGR;
     constexpr int RT = R > 1 ? R - 1 : 1;
     constexpr int NV = 4 * W;  // value byte columns, then 8 + 8 quotient-estimate columns
+    constexpr int CAP = crt_cap(W), ABYTES = CAP * 512;
     static_assert(NV + 16 <= tc::kCrtN, "value and estimate columns fill at most the 128 TMEM columns");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* sbase = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sA = sbase;                                        // [2][128][128 B]
-    uint8_t* sB = sbase + 32768;                                // [2][128][128 B]
-    uint32_t* sR = reinterpret_cast<uint32_t*>(sbase + 65536);  // [R][P][Gc]
-    uint2* sTw = reinterpret_cast<uint2*>(sR + tc::kMaxPrimes * R * 8);  // [P][R-1]
+    uint8_t* sA = sbase;                                        // [CAP/32][128][128 B]
+    uint8_t* sB = sbase + ABYTES;                                  // [CAP/32][128][128 B]
+    uint32_t* sR = reinterpret_cast<uint32_t*>(sbase + 2 * ABYTES);  // [R][CAP][Gc]
+    uint2* sTw = reinterpret_cast<uint2*>(sR + CAP * R * 8);         // [P][R-1]
     __shared__ uint64_t tma_bar, mma_bar;
     __shared__ uint32_t tmem_base;
     __shared__ __align__(16) uint32_t s_q[2 * W];
@@ -456,7 +466,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
     const int begin = int(blockIdx.x) * chunk;
     const int end = min(total, begin + chunk);
 
-    for (int k = tid; k < 2048; k += tc::kCrtThreads) reinterpret_cast<uint4*>(sA)[k] = make_uint4(0, 0, 0, 0);
+    for (int k = tid; k < ABYTES / 16; k += tc::kCrtThreads) reinterpret_cast<uint4*>(sA)[k] = make_uint4(0, 0, 0, 0);
     if (warp == 0) tc::tmem_alloc(&tmem_base, 128);
     if (tid == 0) {
         tc::mbar_init(&tma_bar, 1);
@@ -474,7 +484,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
         const CrtTarget t = w.target(it.x);
         if (!t.use_tma) return;
         const int C = 1 << (LOGC ? LOGC : t.logC), Gc = C < 8 ? C : 8;
-        tc::mbar_expect_tx(&tma_bar, uint32_t(tc::kMaxPrimes * R * Gc) * 4u);  // the whole box, absent primes zero-filled
+        tc::mbar_expect_tx(&tma_bar, uint32_t(CAP * R * Gc) * 4u);  // the whole box, absent primes zero-filled
         tc::tma_load_4d(sR, t.map, it.y * Gc, 0, 0, t.mz, &tma_bar);
     };
     const uint8_t* cur_w = nullptr;  // the product whose tables are in shared memory
@@ -491,7 +501,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
         const int cg = it.y;
         if (t.crt_w != cur_w || t.P != cur_P) {  // the previous item's MMA is complete: B may be rewritten
             const uint4* src = reinterpret_cast<const uint4*>(t.crt_w);
-            for (int q = tid; q < 2048; q += tc::kCrtThreads) reinterpret_cast<uint4*>(sB)[q] = __ldg(src + q);
+            for (int q = tid; q < ABYTES / 16; q += tc::kCrtThreads) reinterpret_cast<uint4*>(sB)[q] = __ldg(src + q);
             for (int q = tid; q < 2 * W; q += tc::kCrtThreads) s_q[q] = t.consts[q];
             for (int q = tid; q <= 2 * t.P; q += tc::kCrtThreads) s_kf[q] = __ldg(t.kfrac + q);
             for (int q = tid; q < t.P; q += tc::kCrtThreads) {
@@ -503,7 +513,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
                 for (int q = tid; q < t.P * RT; q += tc::kCrtThreads)
                     sTw[q] = __ldg(tw_inv + size_t(q / RT) * kNMax + 1 + q % RT);
             if (t.P != cur_P)  // K columns of absent primes must read as zero
-                for (int q = tid; q < 2048; q += tc::kCrtThreads) reinterpret_cast<uint4*>(sA)[q] = make_uint4(0, 0, 0, 0);
+                for (int q = tid; q < ABYTES / 16; q += tc::kCrtThreads) reinterpret_cast<uint4*>(sA)[q] = make_uint4(0, 0, 0, 0);
             cur_w = t.crt_w;
             cur_P = t.P;
             tc::fence_smem_async();
@@ -520,7 +530,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
             const int box = t.P * R * Gc;
             for (int q = tid; q < box; q += tc::kCrtThreads) {
                 const int c = q % Gc, i = (q / Gc) % t.P, r = q / (Gc * t.P);
-                sR[(r * tc::kMaxPrimes + i) * Gc + c] = t.work[size_t(i) * t.n + (size_t(r) << t.logC) + size_t(cg) * Gc + c];
+                sR[(r * CAP + i) * Gc + c] = t.work[size_t(i) * t.n + (size_t(r) << t.logC) + size_t(cg) * Gc + c];
             }
             __syncthreads();
         }
@@ -534,7 +544,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
             const uint32_t p = s_p[i], two_p = 2 * p;
             uint32_t v[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = sR[(r * tc::kMaxPrimes + i) * gc + c];
+            for (int r = 0; r < R; ++r) v[r] = sR[(r * CAP + i) * gc + c];
             const uint2* tw = sTw + i * RT - 1;  // tw[k] = Psi_inv_rev[k], k >= 1
 #pragma unroll
             for (int s = LOGR - 1; s >= 1; --s) {
@@ -576,11 +586,11 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
             // the residue box is free again: fetch the next item's during the MMA and epilogue
             if (k + 1 < end) issue(k + 1);
             const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB);
-            constexpr uint32_t idesc = tc::idesc_u8(tc::kTileM, tc::kCrtN);
+            constexpr uint32_t idesc = tc::idesc_u8(tc::kTileM, NV + 16);
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
+            for (int ks = 0; ks < CAP / 8; ++ks) {
                 const uint32_t off = (ks >> 2) * 16384 + 32 * (ks & 3);
-                tc::mma_u8(tbase, tc::sw128_desc(a0 + off), tc::sw128_desc(b0 + off), idesc, ks > 0);
+                if (CAP == 64 || 8 * ks < t.P) tc::mma_u8(tbase, tc::sw128_desc(a0 + off), tc::sw128_desc(b0 + off), idesc, ks > 0);
             }
             tc::mma_commit(&mma_bar);
         }
@@ -683,9 +693,9 @@ __global__ void __launch_bounds__(tc::kCrtThreads, 2) k3t_crt(const __grid_const
 // shared-memory bytes the kernels above ask for
 constexpr size_t k1t_smem_bytes() { return 1024 + 32768 + 8192 + 16 * kTS * 4; }
 template <int LOGR>
-constexpr size_t k3t_smem_bytes() {
-    return 1024 + 65536 + size_t(tc::kMaxPrimes) * (1 << LOGR) * 8 * 4 +
-           size_t(tc::kMaxPrimes) * ((1 << LOGR) > 1 ? (1 << LOGR) - 1 : 1) * 8;
+constexpr size_t k3t_smem_bytes(int W) {
+    return 1024 + size_t(crt_cap(W)) * 1024 + size_t(crt_cap(W)) * (1 << LOGR) * 8 * 4 +
+           size_t(crt_cap(W)) * ((1 << LOGR) > 1 ? (1 << LOGR) - 1 : 1) * 8;
 }
 
 }  // namespace pm
