@@ -491,8 +491,13 @@ __global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(co
     int cur_P = 0;
     uint32_t tma_phase = 0, mma_phase = 0;
     bool ok = true;
+    // A plan's launch is a programmatic dependent: its CTAs load the first product's tables, then wait
+    // for the row kernel.  A batch's table-driven launch starts with its data there: the first
+    // box is on its way while the tables load (0.8 us a launch).
+    constexpr bool kDependent = std::is_same<Work, PlanCrtWork>::value;
     grid_trigger();
-    if (begin >= end) grid_wait();
+    if (!kDependent || begin >= end) grid_wait();
+    if (!kDependent && tid == 0 && begin < end) issue(begin);
     for (int k = begin; k < end; ++k) {
         const int2 it = w.item(k);
         const CrtTarget t = w.target(it.x);
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(co
             tc::fence_smem_async();
             __syncthreads();
         }
-        if (k == begin) {
+        if (kDependent && k == begin) {
             grid_wait();  // the row kernel's planes, and the output's previous readers
             if (tid == 0) issue(k);
         }
