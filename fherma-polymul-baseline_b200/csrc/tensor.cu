@@ -202,8 +202,8 @@ CUtensorMap coefficient_map(const PlanCore& s, const void* base, uint32_t count)
 // so a box lands in shared memory as [row][prime][column]
 // Residue planes as (column, prime, row, product); a box of box_primes primes lands as
 // [row][box_primes][column] (primes past P read as zero).
-CUtensorMap residue_map(const PlanCore& s, const void* work, uint32_t count, uint32_t box_primes) {
-    const uint32_t C = 1u << s.logC, R = 1u << s.logR, Gc = C < 8 ? C : 8;
+CUtensorMap residue_map(const PlanCore& s, const void* work, uint32_t count, uint32_t box_primes, uint32_t cols = 8) {
+    const uint32_t C = 1u << s.logC, R = 1u << s.logR, Gc = C < cols ? C : cols;
     const cuuint64_t dims[4] = {C, s.P, R, count};
     const cuuint64_t strides[3] = {C * R * 4ull, C * 4ull, s.workspace_bytes};
     const cuuint32_t box[4] = {Gc, box_primes, R, 1};
@@ -364,7 +364,15 @@ void launch_conversion(const PlanCore& s, const uint32_t* a, const uint32_t* b, 
 
 template <int LOGR, int W>
 void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t count, cudaStream_t st) {
-    const int C = 1 << s.logC, Gc = C < 8 ? C : 8;
+    // Tiles of 4 columns for launches whose tiles of 4 are at most one an SM, of bases of more than
+    // 48 primes (at 8 columns more than one and a half rounds of a block's threads).  Whole products
+    // of 868 bits, tiles of 8 / of 4: n = 1024, one 12.8 / 12.0 us, nine 20.1 / 17.5; n = 4096, one 17.4 /
+    // 17.2 (19.4 / 17.8 with other work between the calls), two 20.3 / 18.4; n = 8192, one 21.1 / 18.8.
+    // Past the line: n = 4096, three 20.7 / 21.0; n = 1024, 18 21.5 / 21.6.  Fewer primes: n = 2048 of 640
+    // bits, one 12.3 / 12.7, four 18.8 / 17.7; n = 8192 of 400 bits, one 16.7 / 17.5.
+    const int C = 1 << s.logC;
+    const bool half = LOGR == 4 && s.P > 48 && C >= 8 && int64_t(count) * C <= int64_t(s.sms) * 4;
+    const int Gc = half ? 4 : (C < 8 ? C : 8);
     const int items = int(count) * (C / Gc);
     int ctas = s.sms * k3t_ctas_per_sm(W, s.tune.crt_ctas_per_sm);
     if (ctas > items) ctas = items;
@@ -375,13 +383,15 @@ void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t c
     if (LOGR == 4 && s.logC == 10) kernel = k3t_crt<LOGR, W, PlanCrtWork, 10>;
     if (LOGR == 4 && s.logC == 11) kernel = k3t_crt<LOGR, W, PlanCrtWork, 11>;
     if (LOGR == 4 && s.logC == 12) kernel = k3t_crt<LOGR, W, PlanCrtWork, 12>;
+    if constexpr (LOGR == 4 && W >= 24)  // (49 primes: q of more than 700 bits)
+        if (half) kernel = k3t_crt<LOGR, W, PlanCrtWork, 0, 4>;
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
                "K3T shared memory");
     PlanCrtWork w;
     std::memset(&w.map_res, 0, sizeof w.map_res);
     // rows of fewer than 4 columns, or planes off a 16-byte boundary, cannot be described by a tensor map
     w.use_tma = (C * 4) % 16 == 0 && reinterpret_cast<uintptr_t>(work) % 16 == 0;
-    if (w.use_tma) w.map_res = residue_map(s, work, count, uint32_t(crt_cap(W)));  // a constant row stride in the box
+    if (w.use_tma) w.map_res = residue_map(s, work, count, uint32_t(crt_cap(W)), uint32_t(Gc));  // a constant row stride in the box
     w.work = work;
     w.out = c;
     w.ws_bstride = s.workspace_bytes / 4;
@@ -399,6 +409,7 @@ void launch_k3t(const PlanCore& s, const uint32_t* work, uint32_t* c, uint32_t c
     w.P = int(s.P);
     w.stride = int(s.stride);
     w.count = int(count);
+    w.log_cols = half ? 2 : 3;
     launch_dependent(true, kernel, ctas, tc::kCrtThreads, smem, st, w, s.plane_pc(), s.plane_inv(), s.d_err);
 }
 

@@ -129,7 +129,8 @@ struct PlanCrtWork {
     uint64_t mu_q;
     int sbits, n, logC, P, stride, count, use_tma;
     uint32_t delta;
-    __device__ int lg() const { return logC - min(logC, 3); }  // column groups per row = 2^lg
+    int log_cols = 3;  // columns of a tile = 2^log_cols (at most the row's)
+    __device__ int lg() const { return logC - min(logC, log_cols); }  // column groups per row = 2^lg
     __device__ int total() const { return count << lg(); }
     __device__ int2 item(int k) const { return make_int2(k >> lg(), k & ((1 << lg()) - 1)); }
     __device__ CrtTarget target(int z) const {
@@ -439,7 +440,11 @@ constexpr int k3t_ctas_per_sm(int W, int tuned) { return tuned == 2 ? k3t_min_bl
 
 // LOGC > 0: every item's rows hold 2^LOGC values (a plan's launch at a common ring size), so
 // the tile's column count and the output offsets are constants; 0: read from the item.
-template <int LOGR, int W, class Work, int LOGC = 0>
+// COLS: columns of a tile (rows shorter than that are one tile).  A launch of few products takes
+// tiles of 4: its SMs outnumber its tiles, and the 59 x 8 (prime, column) pairs of a tile of 8
+// are two rounds of the block's 256 threads, those of a tile of 4 one.  The other half of the
+// MMA's 128 rows stays zero.
+template <int LOGR, int W, class Work, int LOGC = 0, int COLS = 8>
 __global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(const __grid_constant__ Work w, const PrimeConst* __restrict__ pcs,
                                                const uint2* __restrict__ tw_inv, uint32_t* __restrict__ err) {
     constexpr int R = 1 << LOGR;
@@ -483,7 +488,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(co
         const int2 it = w.item(k);
         const CrtTarget t = w.target(it.x);
         if (!t.use_tma) return;
-        const int C = 1 << (LOGC ? LOGC : t.logC), Gc = C < 8 ? C : 8;
+        const int C = 1 << (LOGC ? LOGC : t.logC), Gc = C < COLS ? C : COLS;
         tc::mbar_expect_tx(&tma_bar, uint32_t(CAP * R * Gc) * 4u);  // the whole box, absent primes zero-filled
         tc::tma_load_4d(sR, t.map, it.y * Gc, 0, 0, t.mz, &tma_bar);
     };
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(co
         const int2 it = w.item(k);
         const CrtTarget t = w.target(it.x);
         const int logC = LOGC ? LOGC : t.logC;
-        const int C = 1 << logC, Gc = C < 8 ? C : 8;
+        const int C = 1 << logC, Gc = C < COLS ? C : COLS;
         const int cg = it.y;
         if (t.crt_w != cur_w || t.P != cur_P) {  // the previous item's MMA is complete: B may be rewritten
             const uint4* src = reinterpret_cast<const uint4*>(t.crt_w);
@@ -578,8 +583,8 @@ __global__ void __launch_bounds__(tc::kCrtThreads, k3t_min_blocks(W)) k3t_crt(co
             for (int r = 0; r < R; ++r)
                 *reinterpret_cast<uint32_t*>(sA + ka * 16384 + tc::sw128_offset(r * gc + c, kb)) = v[r];
         };
-        if (Gc == 8) {
-            for (int pr = tid; pr < pairs; pr += tc::kCrtThreads) digits(std::integral_constant<int, 8>{}, pr);
+        if (Gc == COLS) {
+            for (int pr = tid; pr < pairs; pr += tc::kCrtThreads) digits(std::integral_constant<int, COLS>{}, pr);
         } else {
             for (int pr = tid; pr < pairs; pr += tc::kCrtThreads) digits(std::integral_constant<int, 0>{}, pr);
         }
