@@ -11,7 +11,7 @@
 //   crt_ctas_per_sm  persistent CTAs of the tensor CRT per SM;
 //   row_persistent   K2 as one CTA per row, or as the persistent kernel that
 //                    stages each row's twiddles once per group and prefetches;
-//   group            products per launch group in batched calls, 4..64 (larger
+//   group            products per launch group in batched calls, 4..128 (larger
 //                    groups amortize each persistent kernel's set-up and tail).
 // Coordinate descent from the defaults, objective = device time per product of
 // a batched call (a change must gain more than 0.3%); results are cached per
