@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
             }
         }
         grid_trigger();
-        grid_wait();  // the coefficients, and the planes' previous readers; the epilogue only follows the MMAs
+        grid_wait();  // the coefficients, and the planes' previous readers
         if (tiles > 0) {
             if (!PLAIN)
                 for (; issued < kFoldTiles && issued < tiles; ++issued)
@@ -308,6 +308,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&empty[pair]);  // this warp's reads of the pair are complete
         };
+        grid_wait();  // so that the bounded waits begin when the producer's do, not while the previous kernel runs
         uint32_t parity = 0;
         for (int u = set; u < 2 * tiles; u += kFoldSets, parity ^= 1u) {
             const int half = u & 1;

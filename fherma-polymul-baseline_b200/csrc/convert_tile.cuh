@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
             tc::bulk_load(sB, conv_w, 32768u, &b_full);
         }
         grid_trigger();
-        grid_wait();  // the coefficients, and the planes' previous readers; the workers only follow this warp
+        grid_wait();  // the coefficients, and the planes' previous readers
         if ((PLAIN || lane == 0) && begin < end) {
             issue(begin, 0);
             if (begin + 1 < end) issue(begin + 1, 1);
@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(tc::kWideThreads, 2) k1w_convert(const __grid_
         const uint32_t taddr = tbase + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(128 * half);
         const int ilo = 32 * half;
         uint32_t ph_mma = 0;
+        grid_wait();  // so that the bounded waits begin when the producer's do, not while the previous kernel runs
         for (int k = begin; k < end; ++k) {
             const TileItem it = w.item(k);
             const ConvTarget t = w.target(it.z, it.poly);

@@ -12,9 +12,10 @@ namespace pm {
 // Programmatic dependent launch.  A kernel launched with that attribute may start before the
 // previous kernel of its stream has finished: it sets up (barriers, tensor memory, constant
 // tables), then grid_wait() holds it until that kernel is complete and its writes are visible.
-// Every CTA waits, so a kernel's completion still implies its predecessors'.  grid_trigger() lets
-// the next kernel start early; a CTA calls it once it holds all it will allocate.  Both do
-// nothing in a plain launch.
+// Every CTA waits, so a kernel's completion still implies its predecessors'; and every thread that
+// waits on an mbarrier afterwards does, so that no bounded wait (mbar_wait) runs against the time a
+// previous kernel takes.  grid_trigger() lets the next kernel start early; a CTA calls it once it
+// holds all it will allocate.  Both do nothing in a plain launch.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
