@@ -206,6 +206,7 @@ struct PlanCore {
 
 void launch_simt(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_t* work,
                  uint32_t count, cudaStream_t st);
+uint32_t default_group(const PlanCore& s);  // products per launch group where no tuning sets it
 uint32_t group_size(const PlanCore& s);
 void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t st, bool early = true);
 void check_device_errors(const PlanCore& s);

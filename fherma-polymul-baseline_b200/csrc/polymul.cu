@@ -415,8 +415,13 @@ void PlanCore::init_tables_only(uint32_t n_, const uint64_t* q64, uint32_t q_lim
     init(n_, q64, q_limbs, coef_limbs_, flags_);
 }
 
+// From kMaxDefaultGroup products on, the plan's buffer is made for its whole default group at once
+// (beyond that many only where their planes take at most kSmallGroupBytes): batches of any such count
+// share it, so a larger one neither moves the buffer that a captured graph points to nor allocates
+// during a capture.
 void PlanCore::ensure_batch_workspace(uint32_t group) {
     if (batch_work_group >= group) return;
+    if (group >= kMaxDefaultGroup) group = std::max(group, default_group(*this));
     cuda_check(cudaStreamSynchronize(stream), "drain plan stream");
     cudaFree(d_batch_work);
     d_batch_work = nullptr;
@@ -651,8 +656,7 @@ void check_device_errors(const PlanCore& s) {
 // bytes.  Products of few residues go in larger groups, as many as keep their planes at 64 MB
 // (half the L2): a launch of 128 of them is mostly its own start and end.  500 products of 200
 // bits at n = 1024 (57 MB): 158 us in four groups of at most 128, 92 us in one.
-uint32_t group_size(const PlanCore& s) {
-    if (s.tune.group) return s.tune.group;
+uint32_t default_group(const PlanCore& s) {
     const size_t budget = size_t(2) << 30;
     size_t g = budget / s.workspace_bytes;
     if (g < 1) g = 1;
@@ -660,6 +664,8 @@ uint32_t group_size(const PlanCore& s) {
         g = std::min<size_t>(kMaxSmallGroup, std::max<size_t>(kMaxDefaultGroup, kSmallGroupBytes / s.workspace_bytes));
     return uint32_t(g);
 }
+
+uint32_t group_size(const PlanCore& s) { return s.tune.group ? s.tune.group : default_group(s); }
 
 void launch_batch(const PlanCore& s, const uint64_t* a, const uint64_t* b, uint64_t* c, uint32_t count,
                   uint32_t group, void* workspace, cudaStream_t st) {

@@ -1,9 +1,9 @@
 """Products on a stream with other work before them.
 
 The library's kernels may start while the kernel before them on the stream still runs and then wait
-for it.  Here that kernel is the caller's own: it lets its dependents start at once and runs for
-longer than the limit of the kernels' bounded waits (1 s), which must not run against it.
-Both conversion kernels, with tensor maps and without, against the oracle."""
+for it: behind a caller's kernel that lets its dependents start at once and outlasts the limit of
+the kernels' bounded waits (1 s), and in captured graphs, whose buffers later calls must leave
+alone.  Against the oracle."""
 import numpy as np
 import pytest
 
@@ -54,3 +54,37 @@ def test_bounded_waits_start_after_the_previous_kernel(cuda, n, bits, limbs, cou
             assert (got[k] == want).all()
         # the plan's error word: no wait gave up
         assert (p.multiply_host(a, b) == want).all()
+
+
+def test_captured_batches_keep_the_plans_workspace(cuda):
+    """A batch larger than the ones before it neither moves the buffer that captured graphs use nor
+    needs a larger one during a capture."""
+    torch = cuda
+    n, bits, limbs = 1024, 200, 4
+    rng = np.random.default_rng(5)
+    q = random_q(rng, bits)
+    few = [uniform_below(rng, q, n, limbs) for _ in range(5)]
+    want = [[oracle.rns_multiply(x, y, q) for y in few] for x in few]
+    pick = [(k % 5, (k // 5) % 5) for k in range(600)]
+    da, db = (torch.from_numpy(np.stack([few[p[s]] for p in pick]).view(np.int64)).cuda() for s in (0, 1))
+    with polymul.Plan(n, q, limbs) as p:
+        def multiply(c):
+            p.multiply_batch(da.data_ptr(), db.data_ptr(), c.data_ptr(), len(c),
+                             stream=torch.cuda.current_stream().cuda_stream)
+
+        outs = [torch.zeros((count, n, limbs), dtype=torch.int64, device="cuda") for count in (128, 600)]
+        multiply(outs[0])
+        torch.cuda.synchronize()
+        graphs = []
+        for c in outs:  # the second is larger than every batch before it
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                multiply(c)
+            graphs.append(g)
+            multiply(torch.zeros_like(outs[1]))
+        for g, c in zip(graphs, outs):
+            c.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            got = c.cpu().numpy().view(np.uint64)
+            assert all((got[k] == want[pick[k][0]][pick[k][1]]).all() for k in range(len(c)))
