@@ -493,7 +493,7 @@ struct BatchCore {
 
     void run(cudaStream_t st) {
         cuda_check(cudaGraphLaunch(graph, st), "batch graph launch");
-        count_launches(1 + row_classes.size() + crt_classes.size());
+        count_launches(fold_classes.size() + row_classes.size() + crt_classes.size());
     }
 };
 
