@@ -135,10 +135,10 @@ Tuning autotune(PlanCore& s, uint32_t reps, double* us_per_product) {
             t.conv_ctas_per_sm = k;
             if (k != best.conv_ctas_per_sm) consider(t);
         }
-        for (int k : {1, 2}) {
+        for (int k = 1; k < k3t_ctas_per_sm(int(s.W), 0); ++k) {  // fewer than the default, as many as fit
             Tuning t = best;
             t.crt_ctas_per_sm = k;
-            if (k != best.crt_ctas_per_sm) consider(t);
+            consider(t);
         }
     }
     for (uint32_t g : {4u, 8u, 16u, 32u, 64u, 128u}) {
@@ -169,7 +169,7 @@ extern "C" int pm_plan_autotune(pm_plan* plan, uint32_t reps, pm_tuning* chosen)
         if (chosen) {
             chosen->row_radix = 1u << t.row_radix_log;
             chosen->conv_ctas_per_sm = uint32_t(t.conv_ctas_per_sm);
-            chosen->crt_ctas_per_sm = uint32_t(t.crt_ctas_per_sm);
+            chosen->crt_ctas_per_sm = uint32_t(pm::k3t_ctas_per_sm(int(plan->core.W), t.crt_ctas_per_sm));
             chosen->group = t.group;
             chosen->row_persistent = t.row_persistent ? 1u : 0u;
             chosen->conv_whole_basis = t.conv_whole_basis ? 1u : 0u;

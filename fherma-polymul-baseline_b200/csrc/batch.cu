@@ -219,7 +219,7 @@ struct BatchCore {
     cudaGraphExec_t graph = nullptr;
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> events;
-    int crt_ctas_per_sm = 2;  // persistent grid size (autotuned)
+    int crt_ctas_per_sm = 0;  // persistent grid size (0: as many as fit; autotuned)
 
     ~BatchCore() {
         cudaSetDevice(device);
@@ -484,9 +484,11 @@ struct BatchCore {
                 if (k == cur || rc.logC < 10) continue;  // the warp kernel's passes are fixed
                 attempt([&] { rc.radix_log = k; }, [&] { rc.radix_log = cur; });
             }
-        {
+        for (int k : {1, 2}) {
+            const bool differs = std::any_of(crt_classes.begin(), crt_classes.end(),
+                                             [&](const CrtClass& cc) { return k < k3t_ctas_per_sm(cc.W, 0); });
             const int old = crt_ctas_per_sm;
-            attempt([&] { crt_ctas_per_sm = 1; }, [&] { crt_ctas_per_sm = old; });
+            if (differs) attempt([&] { crt_ctas_per_sm = k; }, [&] { crt_ctas_per_sm = old; });
         }
         return best;
     }

@@ -115,7 +115,7 @@ constexpr uint32_t kMaxGroup = 256;
 struct Tuning {
     int row_radix_log = 4;   // K2 register-pass radix: 2, 3 or 4 (radix 4, 8, 16; 16 in the persistent kernel)
     int conv_ctas_per_sm = 3;  // K1T persistent CTAs per SM (up to four fit; three measured fastest)
-    int crt_ctas_per_sm = 2;   // K3T persistent CTAs per SM
+    int crt_ctas_per_sm = 0;   // K3T persistent CTAs per SM; 0: as many as fit (k3t_ctas_per_sm)
     bool row_persistent = true;  // K2P (rows of C >= 1024) and K2W (16 .. 512) instead of K2
     bool conv_whole_basis = true;  // tensor conversion: one pass of a tile over every prime (K1W) or per group (K1T)
     uint32_t group = 0;        // products per launch group in batches (0: up to ~2 GB of residues, <= 128)
@@ -206,6 +206,7 @@ struct PlanCore {
 
 void launch_simt(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_t* work,
                  uint32_t count, cudaStream_t st);
+int k3t_ctas_per_sm(int W, int tuned);   // CTAs per SM of a K3T launch: the tuning's, or (0) as many as fit
 uint32_t default_group(const PlanCore& s);  // products per launch group where no tuning sets it
 uint32_t group_size(const PlanCore& s);
 void launch_rows(const PlanCore& s, uint32_t* work, uint32_t count, cudaStream_t st, bool early = true);

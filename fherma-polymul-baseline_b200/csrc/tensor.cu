@@ -82,6 +82,8 @@ std::vector<uint8_t> fold_image(const DeviceBasis& B, int f) {
 }
 }  // namespace
 
+int k3t_ctas_per_sm(int W, int tuned) { return tuned ? tuned : k3t_min_blocks(W); }
+
 void tensor_init(PlanCore& s) {
     if (uint32_t(s.P) * 4 > uint32_t(tc::kCrtK)) throw Failure(PM_ERR_UNSUPPORTED, "prime basis too large for the CRT tile");
     if (4 * s.W + 16 > uint32_t(tc::kCrtN)) throw Failure(PM_ERR_UNSUPPORTED, "q too wide for the CRT tile");

@@ -435,8 +435,6 @@ __device__ __forceinline__ void add1_carry(uint32_t& a, uint32_t b, uint32_t& cy
 // 37.2 -> 31.3 us; an uneven batch of 200 to 868 bits, whole, 401 -> 390.
 constexpr int crt_cap(int W) { return W <= 12 ? 32 : 64; }
 constexpr int k3t_min_blocks(int W) { return W <= 12 ? 3 : 2; }
-// CTAs per SM of a launch: the tuning's default of two stands for as many as fit
-constexpr int k3t_ctas_per_sm(int W, int tuned) { return tuned == 2 ? k3t_min_blocks(W) : tuned; }
 
 // LOGC > 0: every item's rows hold 2^LOGC values (a plan's launch at a common ring size), so
 // the tile's column count and the output offsets are constants; 0: read from the item.

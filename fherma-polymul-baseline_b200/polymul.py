@@ -246,8 +246,12 @@ class Plan:
         check(lib().pm_plan_autotune(self._h, reps, ctypes.byref(t)))
         return {name: getattr(t, name) for name, _ in Tuning._fields_}
 
-    def set_tuning(self, row_radix=16, conv_ctas_per_sm=3, crt_ctas_per_sm=2, group=0, row_persistent=1,
+    def set_tuning(self, row_radix=16, conv_ctas_per_sm=3, crt_ctas_per_sm=None, group=0, row_persistent=1,
                    conv_whole_basis=1):
+        """Launch shapes; what is not given is as in an untuned plan (crt_ctas_per_sm: as many as fit,
+        three for q of up to 384 bits, else two)."""
+        if crt_ctas_per_sm is None:
+            crt_ctas_per_sm = 3 if self.q.bit_length() <= 384 else 2
         t = Tuning(row_radix, conv_ctas_per_sm, crt_ctas_per_sm, group, row_persistent, conv_whole_basis, 0.0)
         check(lib().pm_plan_set_tuning(self._h, ctypes.byref(t)))
 

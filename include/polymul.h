@@ -97,7 +97,8 @@ typedef struct {
     uint32_t row_radix;         /* radix of the row NTT register passes: 4, 8 or 16 (16: rows of >= 1024
                                    values in the persistent kernel; other rows then use 8) */
     uint32_t conv_ctas_per_sm;  /* persistent CTAs of the tensor conversion per SM, 1..8 */
-    uint32_t crt_ctas_per_sm;   /* persistent CTAs of the tensor CRT per SM, 1..4 */
+    uint32_t crt_ctas_per_sm;   /* persistent CTAs of the tensor CRT per SM, 1..4 (an untuned plan: as many as
+                                   fit, three for q of up to 384 bits, else two) */
     uint32_t group;             /* products per launch group in batched calls (0: up to ~2 GB of residues and
                                    128 products, or more in 64 MB of residues; at most 256) */
     uint32_t row_persistent;    /* 1: the kernels that stage a row's twiddles once per group of products (rows
