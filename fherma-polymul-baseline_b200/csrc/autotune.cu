@@ -11,14 +11,17 @@
 //   crt_ctas_per_sm  persistent CTAs of the tensor CRT per SM;
 //   row_persistent   K2 as one CTA per row, or as the persistent kernel that
 //                    stages each row's twiddles once per group and prefetches;
-//   group            products per launch group in batched calls, 4..128 (larger
-//                    groups amortize each persistent kernel's set-up and tail).
+//   group            products per launch group in batched calls, 4..128, against the
+//                    default, which may be larger (larger groups amortize each
+//                    persistent kernel's set-up and tail).
 // Coordinate descent from the defaults, objective = device time per product of
-// a batched call (a change must gain more than 0.3%); results are cached per
+// a batched call of as many products as the default group holds (a change must
+// gain more than 0.3%; what would launch the same is not tried); results are cached per
 // (n, bits(q), coef_limbs, path) for the life of the process, so later plans
 // with the same shape reuse them.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -65,10 +68,10 @@ Tuning autotune(PlanCore& s, uint32_t reps, double* us_per_product) {
         }
     }
     if (reps == 0) reps = 3;
-    // a batch big enough for the largest group tried, capped at ~4 GB of buffers
+    // a batch big enough for the largest group tried and the default one, capped at ~4 GB of buffers
     const size_t per = 3 * s.io_bytes + s.workspace_bytes;
     uint32_t count = uint32_t((size_t(4096) << 20) / per);
-    count = count < 1 ? 1 : (count > kMaxDefaultGroup ? kMaxDefaultGroup : count);
+    count = std::max(1u, std::min(count, std::max(kMaxDefaultGroup, default_group(s))));
     Scratch sc;
     cuda_check(cudaStreamCreateWithFlags(&sc.st, cudaStreamNonBlocking), "autotune stream");
     cuda_check(cudaEventCreate(&sc.e0), "autotune event");
@@ -124,7 +127,7 @@ Tuning autotune(PlanCore& s, uint32_t reps, double* us_per_product) {
         }
     }
     if (s.flags & PM_CONVERT_TENSOR) {
-        {
+        if (!s.plain_rows) {  // (rows without tensor maps: the same kernels either way)
             Tuning t = best;
             t.conv_whole_basis = !best.conv_whole_basis;
             consider(t);
@@ -143,6 +146,7 @@ Tuning autotune(PlanCore& s, uint32_t reps, double* us_per_product) {
     }
     for (uint32_t g : {4u, 8u, 16u, 32u, 64u, 128u}) {
         if (g > count) break;
+        if (g == std::min(count, default_group(s))) continue;  // the launches already timed
         Tuning t = best;
         t.group = g;
         consider(t);

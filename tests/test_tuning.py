@@ -1,4 +1,5 @@
-"""Launch shapes as asked for: the grids that a captured product's kernels have under each tuning."""
+"""Launch shapes as asked for (the grids that a captured product's kernels have under each tuning), and
+the autotuner's choice among those that differ."""
 import ctypes
 
 import numpy as np
@@ -55,3 +56,17 @@ def test_crt_ctas_per_sm_is_what_was_asked_for(cuda, bits, limbs, fit):
         chosen = p.autotune()
         p.set_tuning(crt_ctas_per_sm=chosen["crt_ctas_per_sm"], group=count)
         assert _crt_grid(torch, p, count, limbs) == chosen["crt_ctas_per_sm"] * sms
+
+
+def test_autotuner_weighs_the_default_group(cuda):
+    """Launch shapes that only repeat the default's are not picked: with the default group of 585 small
+    products (one launch instead of five, half the time), with a default of 128, and with the
+    conversion of rows without tensor maps, which has one form."""
+    rng = np.random.default_rng(9)
+    with polymul.Plan(1024, random_q(rng, 200), 4) as p:
+        default = p.batch_workspace_size(5000)
+        assert p.autotune()["group"] == 0
+        assert p.batch_workspace_size(5000) == default
+    with polymul.Plan(16384, random_q(rng, 517), 9) as p:
+        chosen = p.autotune()
+        assert chosen["group"] != 128 and chosen["conv_whole_basis"] == 1
