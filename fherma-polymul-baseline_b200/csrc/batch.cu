@@ -7,7 +7,9 @@
 //   conversion items  (product, polynomial, column group) per number of folded
 //                     column stages (three, two or one, by the product's basis) --
 //                     one persistent launch of k1f_convert per class, each on its
-//                     share of the SMs;
+//                     share of the SMs; in batches of few tiles (product, prime
+//                     group, polynomial, column group) ordered prime group first --
+//                     one persistent launch of k1t_convert;
 //   row items         (product, prime, first row) per ring size class -- one
 //                     launch per class: the persistent k2p_rows for rows of
 //                     1024 values or more (items prime/row first, so a CTA
@@ -54,6 +56,36 @@ struct TableFoldWork {
         return ConvTarget{maps + 3 * z + poly, 0, work + d.ws_off, d.n, d.logC, d.P};
     }
 };
+
+// the same work by K1T: (product, prime group, polynomial, column group) items of every class
+struct TableConvWork {
+    const uint4* items;
+    int nitems;
+    const BatchProduct* prod;
+    const CUtensorMap* maps;
+    uint32_t* work;
+    __device__ int total() const { return nitems; }
+    __device__ ConvItem item(int k) const {
+        const uint4 v = items[k];
+        return ConvItem{int(v.x), int(v.y), int(v.z), int(v.w)};
+    }
+    __device__ ConvTarget target(int z, int poly) const {
+        const BatchProduct& d = prod[z];
+        return ConvTarget{maps + 3 * z + poly, 0, work + d.ws_off, d.n, d.logC, d.P};
+    }
+    __device__ int2 range(int b, int grid) const {  // contiguous runs of the table
+        const int chunk = (nitems + grid - 1) / grid;
+        return make_int2(min(nitems, b * chunk), min(nitems, (b + 1) * chunk));
+    }
+};
+
+// Tiles of 128 coefficients an SM up to which a batch converts by K1T.  K1F's CTAs fill an SM and load
+// 128 KB of weights each before their first tile, a launch per class; K1T is one launch of small CTAs,
+// three an SM, that share a tile's primes out.  Whole batches, K1T / K1F: one product of 256, 868 bits,
+// 16.4 / 22.6 us; eight of 1024 (128 tiles) 20.6 / 24.6; four of 192 .. 590 bits (312) 27.8 / 33.2;
+// two of 8192 (256) 28.7 / 28.7.  Past the line either: four of 8192, 400 bits (512), 28.7 / 26.7;
+// eight of 4096, 600 bits (512), 30.8 / 32.8; 64 of 1024 (1024) 55.4 / 53.3.
+constexpr int kBatchTilesPerSm = 3;
 
 // rows of one size class from a table of (product, prime, first row) items
 struct TableRowWork {
@@ -201,6 +233,7 @@ struct BatchCore {
     uint4* d_row_items = nullptr;
     uint2* d_crt_items = nullptr;
     uint32_t* d_err = nullptr;
+    int conv_items = 0;  // of K1T, or none
     struct FoldClass {
         int f, count, ctas, qbytes;
         size_t offset;  // into d_conv_items
@@ -219,7 +252,8 @@ struct BatchCore {
     cudaGraphExec_t graph = nullptr;
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> events;
-    int crt_ctas_per_sm = 0;  // persistent grid size (0: as many as fit; autotuned)
+    int conv_ctas_per_sm = 3;  // persistent grid size of K1T (autotuned)
+    int crt_ctas_per_sm = 0;   // of the CRT (0: as many as fit; autotuned)
 
     ~BatchCore() {
         cudaSetDevice(device);
@@ -254,6 +288,14 @@ struct BatchCore {
             cuda_check(cudaStreamWaitEvent(st0, e, 0), "batch join");
         };
         std::vector<cudaStream_t> used;
+        if (conv_items) {
+            cuda_check(cudaFuncSetAttribute(k1t_convert<4, TableConvWork>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            int(k1t_smem_bytes())),
+                       "batch conversion shared memory");
+            const TableConvWork w{d_conv_items, conv_items, d_prod, d_maps, d_work};
+            k1t_convert<4, TableConvWork><<<std::min(conv_items, sms * conv_ctas_per_sm), tc::kConvThreads,
+                                            k1t_smem_bytes(), st0>>>(w, B.d_pc, B.d_conv_weights, B.d_tw_fwd, d_err);
+        }
         for (size_t k = 0; k < fold_classes.size(); ++k) {
             const FoldClass& fc = fold_classes[k];
             cudaStream_t s = fork(k);
@@ -330,18 +372,22 @@ struct BatchCore {
         cuda_check(cudaMalloc(&d_work, ws * 4), "batch workspace");
         cuda_check(cudaMalloc(&d_err, 4), "batch error word");
         cuda_check(cudaMemset(d_err, 0, 4), "batch error word");
+        const int sms = sm_count_dev();
+        size_t tiles128 = 0;
+        for (auto& p : plans) tiles128 += 2 * size_t(p->n) / tc::kTileM;
+        const bool fold = tiles128 > size_t(sms) * kBatchTilesPerSm;  // K1F, or K1T
         // tensor maps: a, b coefficient bytes and residue planes of each product
         std::vector<CUtensorMap> maps(3 * size_t(cnt));
         for (uint32_t z = 0; z < cnt; ++z) {
             const PlanCore& p = *plans[z];
             const cuuint64_t C = 1ull << p.logC, R = 1ull << p.logR, sb = p.stride * 4ull;
             const cuuint32_t Gc = cuuint32_t(C < 8 ? C : 8);
-            const int f = fold_stages(int(p.P), int(p.logC));  // at least one: n >= 256
+            const int f = fold ? fold_stages(int(p.P), int(p.logC)) : 0;  // K1F: at least one, as n >= 256
             const cuuint64_t cdims[4] = {sb, C, R, 1};
             const cuuint64_t cstr[3] = {sb, sb * C, sb * C * R};
-            const cuuint32_t cbox[4] = {256u >> f, 8u << f, 16u >> f, 1};
+            const cuuint32_t cbox[4] = {fold ? 256u >> f : 128u, 8u << f, 16u >> f, 1};
             const CUtensorMapSwizzle swizzle =
-                f == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : (f == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+                f <= 1 ? CU_TENSOR_MAP_SWIZZLE_128B : (f == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
             maps[3 * z] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_a + io_off[z], cdims, cstr, cbox, swizzle);
             maps[3 * z + 1] = encode(CU_TENSOR_MAP_DATA_TYPE_UINT8, d_b + io_off[z], cdims, cstr, cbox, swizzle);
             // box lands as [row][32 or 64 primes][column]: a constant row stride (primes past P read as zero)
@@ -352,10 +398,19 @@ struct BatchCore {
                                      CU_TENSOR_MAP_SWIZZLE_NONE);
         }
         // work tables
+        std::vector<uint4> conv;
+        for (int pg = 0; pg < 4 && !fold; ++pg)
+            for (uint32_t z = 0; z < cnt; ++z) {
+                const PlanCore& p = *plans[z];
+                if (pg * 16 >= int(p.P)) continue;
+                for (uint32_t poly = 0; poly < 2; ++poly)
+                    for (uint32_t cg = 0; cg < (1u << p.logC) / 8; ++cg) conv.push_back(make_uint4(z, pg, poly, cg));
+            }
+        conv_items = int(conv.size());
         std::map<int, std::vector<uint4>> conv_by_f;
         std::map<int, int> qbytes_by_f;
         size_t tiles = 0;
-        for (uint32_t z = 0; z < cnt; ++z) {
+        for (uint32_t z = 0; z < cnt && fold; ++z) {
             const PlanCore& p = *plans[z];
             const int f = fold_stages(int(p.P), int(p.logC));
             const uint32_t groups = (1u << p.logC) / (8u << f);
@@ -364,8 +419,6 @@ struct BatchCore {
             qbytes_by_f[f] = std::max(qbytes_by_f[f], int((p.qbits + 7) / 8));
             tiles += 2 * size_t(groups);
         }
-        std::vector<uint4> conv;
-        const int sms = sm_count_dev();
         for (auto& [f, items] : conv_by_f) {
             // a CTA fills an SM: the classes run side by side on shares of them by their tiles
             const int share = int(size_t(sms) * items.size() / tiles);
@@ -484,6 +537,11 @@ struct BatchCore {
                 if (k == cur || rc.logC < 10) continue;  // the warp kernel's passes are fixed
                 attempt([&] { rc.radix_log = k; }, [&] { rc.radix_log = cur; });
             }
+        for (int k : {2, 3, 4}) {
+            const int old = conv_ctas_per_sm;
+            if (k == old || !conv_items) continue;
+            attempt([&] { conv_ctas_per_sm = k; }, [&] { conv_ctas_per_sm = old; });
+        }
         for (int k : {1, 2}) {
             const bool differs = std::any_of(crt_classes.begin(), crt_classes.end(),
                                              [&](const CrtClass& cc) { return k < k3t_ctas_per_sm(cc.W, 0); });
@@ -495,7 +553,7 @@ struct BatchCore {
 
     void run(cudaStream_t st) {
         cuda_check(cudaGraphLaunch(graph, st), "batch graph launch");
-        count_launches(fold_classes.size() + row_classes.size() + crt_classes.size());
+        count_launches((conv_items ? 1 : fold_classes.size()) + row_classes.size() + crt_classes.size());
     }
 };
 

@@ -5,7 +5,7 @@
 // each one is and where its product's data lives:
 //   PlanConvWork / PlanCrtWork   `count` products of one plan, items computed
 //                                from the index (maps are kernel parameters);
-//   TableCrtWork                 products of different n and q (an uneven
+//   TableConvWork / TableCrtWork products of different n and q (an uneven
 //                                batch), items and per-product descriptors read
 //                                from device tables (maps in global memory).
 // Each CTA takes a contiguous chunk of items, so the operand tables it keeps in
