@@ -419,12 +419,20 @@ struct BatchCore {
             qbytes_by_f[f] = std::max(qbytes_by_f[f], int((p.qbits + 7) / 8));
             tiles += 2 * size_t(groups);
         }
+        // a CTA fills an SM: the classes run side by side on shares of them by their tiles; the
+        // largest takes what the others leave, so that no CTA waits for a second round
+        int left = sms;
+        size_t largest = 0;
         for (auto& [f, items] : conv_by_f) {
-            // a CTA fills an SM: the classes run side by side on shares of them by their tiles
-            const int share = int(size_t(sms) * items.size() / tiles);
-            const int ctas = std::min(int(items.size()), std::max(1, share));
+            const int ctas = std::min(int(items.size()), std::max(1, int(size_t(sms) * items.size() / tiles)));
             fold_classes.push_back(FoldClass{f, int(items.size()), ctas, qbytes_by_f[f], conv.size()});
             conv.insert(conv.end(), items.begin(), items.end());
+            left -= ctas;
+            if (items.size() > size_t(fold_classes[largest].count)) largest = fold_classes.size() - 1;
+        }
+        if (fold) {
+            FoldClass& fc = fold_classes[largest];
+            fc.ctas = std::min(fc.count, fc.ctas + left);
         }
         std::map<int, std::vector<uint4>> rows_by_c;
         for (uint32_t z = 0; z < cnt; ++z) {
