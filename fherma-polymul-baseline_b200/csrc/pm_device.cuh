@@ -641,13 +641,13 @@ __global__ void __launch_bounds__(256) k3_cols_crt(const uint32_t* __restrict__ 
             const bool upper = (r >> bit) & 1;
             const uint32_t other = __shfl_xor_sync(mask, v, 1 << bit);
             if (!upper) {
-                v = csub(v + other, pc.two_p);
+                v = csub_pair(v + other, pc.two_p);
             } else {
                 const uint2 w = __ldg(tw + (1 << s) + (r >> (logR - s)));
                 v = shoup_mul(other - v + pc.two_p, w, pc.p);
             }
         }
-        const uint32_t ti = csub(shoup_mul(v, __ldg(scale + i), pc.p), pc.p);
+        const uint32_t ti = csub_pair(shoup_mul(v, __ldg(scale + i), pc.p), pc.p);
         uint32_t m[W];
 #pragma unroll
         for (int k = 0; k < W; ++k) m[k] = s_mq[i * W + k];
