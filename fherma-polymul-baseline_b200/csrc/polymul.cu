@@ -301,7 +301,8 @@ void PlanCore::init(uint32_t n_, const uint64_t* q64, uint32_t q_limbs, uint32_t
     // describe) by the conversion kernels' plain-row forms, which take rows of 16 columns or more
     // (n >= 256).  60 products of 517 bits (9 limbs) at n = 4096: 396 us by the plain method, 135 us so.
     plain_rows = false;
-    if (!(flags_ & (PM_CONVERT_TENSOR | PM_CONVERT_SIMT | PM_WIDE_NTT)) && (coef_limbs_ % 2 == 0 || n_ >= 256)) {
+    if (!(flags_ & (PM_CONVERT_TENSOR | PM_CONVERT_SIMT | PM_WIDE_NTT)) &&
+        (coef_limbs_ % 2 == 0 || (n_ >= 256 && !(flags_ & PM_QUARTIC)))) {
         flags_ |= PM_CONVERT_TENSOR;
         plain_rows = coef_limbs_ % 2 != 0;
     }

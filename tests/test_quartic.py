@@ -61,3 +61,10 @@ def test_quartic_refuses_what_it_does_not_cover(cuda):
     with pytest.raises(polymul.PolymulError) as e:
         polymul.Plan(1024, FHERMA_Q, coef_limbs=14, quartic=True, tensor=False)
     assert e.value.status == polymul.PM_ERR_INVALID
+
+
+@pytest.mark.parametrize("n", [128, 1024])
+def test_quartic_refuses_odd_limbs_as_off_the_tensor_path(cuda, n):
+    with pytest.raises(polymul.PolymulError) as e:
+        polymul.Plan(n, FHERMA_Q, coef_limbs=15, quartic=True)
+    assert e.value.status == polymul.PM_ERR_INVALID
