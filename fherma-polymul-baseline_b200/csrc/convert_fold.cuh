@@ -142,8 +142,19 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
     if constexpr (PLAIN)  // the bytes past the copied words stay zero
         for (int k = tid; k < kFoldTiles * kFoldTileBytes / 16; k += k1f_threads(PLAIN))
             reinterpret_cast<uint4*>(sX)[k] = make_uint4(0, 0, 0, 0);
-    if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
-    if (tid == 0) {
+    if (warp == 0) {
+        tc::tmem_alloc(&tmem_base, 512);
+        grid_trigger();
+    }
+    auto issue = [&](int kk) {
+        const TileItem it = w.item(begin + kk);
+        const ConvTarget t = w.target(it.z, it.poly);
+        const int b = kk % kFoldTiles;
+        tc::mbar_expect_tx(&tma_full[b], uint32_t(kFoldTileBytes));
+        for (int h = 0; h < F; ++h)
+            tc::tma_load_4d(sX + b * kFoldTileBytes + h * BOX, t.map, 0, it.cg * COLS, h * J, t.mz, &tma_full[b]);
+    };
+    if (tid == 32 * 4 * kFoldSets) {
         for (int b = 0; b < kFoldTiles; ++b) {
             tc::mbar_init(&tma_full[b], PLAIN ? 32 * kFoldLoaders : 1);
             tc::mbar_init(&done[b], 1);
@@ -154,6 +165,22 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
         }
         tc::mbar_init(&w_full, 1);
         s_abort = 0;
+        tc::fence_smem_async();
+        if (tiles > 0) {
+            tc::mbar_expect_tx(&w_full, kFoldWeightBytes);
+            for (uint32_t o = 0; o < kFoldWeightBytes; o += 32768) tc::bulk_load(sW + o, weights + o, 32768u, &w_full);
+        }
+    }
+    // Every warp waits for the previous kernel (the coefficients, and the planes' previous readers)
+    // before its first bounded wait.  Here and not in the epilogue's branch: a wait (or, with tensor
+    // maps, a barrier) between here and its loop took registers from the 128 of a thread, 700 -> 729 us for 128
+    // products at n = 32768.  Rows without tensor maps: the warps that load wait below, all others meet
+    // them at a barrier (60 products of 517 bits at n = 4096, whole: 125.6 us with no wait, 126.4 with a
+    // wait in each branch, 124.7 so).
+    if (!PLAIN) {
+        grid_wait();
+        if (tid == 32 * 4 * kFoldSets)
+            for (int kk = 0; kk < kFoldTiles && kk < tiles; ++kk) issue(kk);
     }
     tc::fence_smem_async();
     tc::fence_before();
@@ -164,33 +191,19 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
 
     if (warp == 4 * kFoldSets) {
         // --------------------- MMAs (and the tiles' TMA loads) ----------------
-        auto issue = [&](int kk) {
-            const TileItem it = w.item(begin + kk);
-            const ConvTarget t = w.target(it.z, it.poly);
-            const int b = kk % kFoldTiles;
-            tc::mbar_expect_tx(&tma_full[b], uint32_t(kFoldTileBytes));
-            for (int h = 0; h < F; ++h)
-                tc::tma_load_4d(sX + b * kFoldTileBytes + h * BOX, t.map, 0, it.cg * COLS, h * J, t.mz, &tma_full[b]);
-        };
         auto wait = [&](uint64_t* bar, uint32_t parity) {
             const bool arrived = __all_sync(0xffffffffu, tc::mbar_wait(bar, parity));
             ok = ok && arrived;
             return arrived;
         };
+        if (PLAIN) {
+            grid_wait();
+            __syncthreads();
+        }
         int issued = 0, seen = 0, committed = 0;  // tiles requested, seen complete, given to the tensor cores
         bool w_pending = false;
         if (tiles > 0) {
-            if (lane == 0) {
-                tc::mbar_expect_tx(&w_full, kFoldWeightBytes);
-                for (uint32_t o = 0; o < kFoldWeightBytes; o += 32768) tc::bulk_load(sW + o, weights + o, 32768u, &w_full);
-            }
-        }
-        grid_trigger();
-        grid_wait();  // the coefficients, and the planes' previous readers
-        if (tiles > 0) {
-            if (!PLAIN)
-                for (; issued < kFoldTiles && issued < tiles; ++issued)
-                    if (lane == 0) issue(issued);
+            if (!PLAIN) issued = min(kFoldTiles, tiles);
             w_pending = !wait(&w_full, 0);
         }
         for (int kk = 0; kk < tiles && ok; ++kk) {
@@ -250,7 +263,8 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
                 tc::mbar_arrive(&tma_full[kk % kFoldTiles]);
             };
             int loaded = 0;
-            grid_wait();  // the coefficients
+            grid_wait();
+            __syncthreads();
             for (int kk = 0; kk < tiles; ++kk, ++loaded) {
                 const int b = kk % kFoldTiles;
                 if (kk >= kFoldTiles)  // the MMAs have read the buffer's last tile
@@ -284,6 +298,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
         }
     } else {
         // ------------------------------ epilogue ------------------------------
+        if (PLAIN) __syncthreads();
         const int set = warp >> 2;
         const int m = tid & 127;  // TMEM lane: block h of rows, prime i
         const int i = m % PMAX, h = m / PMAX;
@@ -308,7 +323,6 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&empty[pair]);  // this warp's reads of the pair are complete
         };
-        grid_wait();  // so that the bounded waits begin when the producer's do, not while the previous kernel runs
         uint32_t parity = 0;
         for (int u = set; u < 2 * tiles; u += kFoldSets, parity ^= 1u) {
             const int half = u & 1;
