@@ -66,12 +66,11 @@ struct PlanFoldWork {
     uint32_t* work;
     size_t ws_bstride;
     int n, logC, P, count;
-    int poly_only, log_groups;  // column groups per row = 2^log_groups
+    int log_groups;  // column groups per row = 2^log_groups
     PlainRows plain;            // (the form that loads rows without tensor maps)
-    __device__ int total() const { return count << (log_groups + (poly_only < 0 ? 1 : 0)); }
+    __device__ int total() const { return count << (log_groups + 1); }
     __device__ TileItem item(int k) const {
         const int g = log_groups, cg = k & ((1 << g) - 1);
-        if (poly_only >= 0) return TileItem{k >> g, poly_only, cg};
         return TileItem{k >> (g + 1), (k >> g) & 1, cg};
     }
     __device__ ConvTarget target(int z, int poly) const {

@@ -312,14 +312,13 @@ int plan_fold(const PlanCore& s, const uint32_t* work) {
 
 template <int LOGF>
 void launch_k1f(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
-                cudaStream_t st, int poly_only) {
+                cudaStream_t st) {
     PlanFoldWork w;
-    w.poly_only = poly_only;
     if (s.plain_rows) {
         w.plain = plain_rows(s, a, b, 256 >> LOGF);
     } else {
-        w.map_a = fold_map(s, poly_only == 1 ? b : a, count, LOGF);
-        w.map_b = poly_only == 0 ? w.map_a : fold_map(s, b, count, LOGF);
+        w.map_a = fold_map(s, a, count, LOGF);
+        w.map_b = fold_map(s, b, count, LOGF);
     }
     w.work = work;
     w.ws_bstride = s.workspace_bytes / 4;
@@ -328,29 +327,29 @@ void launch_k1f(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_
     w.P = int(s.P);
     w.count = int(count);
     w.log_groups = int(s.logC) - (LOGF + 3);
-    const int items = int(count) * (poly_only < 0 ? 2 : 1) << w.log_groups;
+    const int items = int(count) * 2 << w.log_groups;
     auto kernel = s.plain_rows ? k1f_convert<LOGF, PlanFoldWork, true> : k1f_convert<LOGF, PlanFoldWork>;
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k1f_smem_bytes())),
                "K1F shared memory");
-    launch_dependent(poly_only < 0, kernel, std::min(items, s.sms), k1f_threads(s.plain_rows), k1f_smem_bytes(), st, w, s.basis->d_pc,
+    launch_dependent(true, kernel, std::min(items, s.sms), k1f_threads(s.plain_rows), k1f_smem_bytes(), st, w, s.basis->d_pc,
                      s.basis->d_fold_weights + (LOGF - 1) * size_t(kFoldWeightBytes), s.basis->d_tw_fwd,
                      int((s.qbits + 7) / 8), s.d_err);
 }
 
-// Conversion of both polynomials (poly_only < 0) or of one, by the folding kernel or K1W.  K1F
-// loads 128 KB of weights per CTA before its first tile, against K1W's 32 KB and twice the CTAs:
-// K1W stays where it finishes in two rounds (592 tiles of 128 coefficients on 148 SMs).  Measured
-// on either side, whole products (868 bits unless said): n = 32768, one 38.8 us by K1W / 39.2 by
-// K1F, two 64.6 / 64.3, eight 189.7 / 183.9; n = 1024, one 17.1 / 19.4, 32 of 200 bits (512 tiles)
-// 19.5 / 20.0; n = 4096, 16 of 200 bits (1024 tiles) 27.4 / 25.0.
+// Conversion of both polynomials (poly_only < 0) by the folding kernel or K1W, or of one by K1W (at
+// n <= 65536 one has at most 512 tiles).  K1F loads 128 KB of weights per CTA before its first tile,
+// against K1W's 32 KB and twice the CTAs: K1W stays where it finishes in two rounds (592 tiles of 128
+// coefficients on 148 SMs).  Measured on either side, whole products (868 bits unless said): n = 32768,
+// one 38.8 us by K1W / 39.2 by K1F, two 64.6 / 64.3, eight 189.7 / 183.9; n = 1024, one 17.1 / 19.4,
+// 32 of 200 bits (512 tiles) 19.5 / 20.0; n = 4096, 16 of 200 bits (1024 tiles) 27.4 / 25.0.
 template <int LOGR>
 void launch_whole_basis(const PlanCore& s, const uint32_t* a, const uint32_t* b, uint32_t* work, uint32_t count,
                         cudaStream_t st, int poly_only = -1) {
-    const size_t tiles = size_t(count) * (poly_only < 0 ? 2 : 1) * s.n / tc::kTileM;
-    switch (LOGR == 4 && tiles > size_t(s.sms) * 4 ? plan_fold(s, work) : 0) {
-        case 1: return launch_k1f<1>(s, a, b, work, count, st, poly_only);
-        case 2: return launch_k1f<2>(s, a, b, work, count, st, poly_only);
-        case 3: return launch_k1f<3>(s, a, b, work, count, st, poly_only);
+    const size_t tiles = size_t(count) * 2 * s.n / tc::kTileM;
+    switch (LOGR == 4 && poly_only < 0 && tiles > size_t(s.sms) * 4 ? plan_fold(s, work) : 0) {
+        case 1: return launch_k1f<1>(s, a, b, work, count, st);
+        case 2: return launch_k1f<2>(s, a, b, work, count, st);
+        case 3: return launch_k1f<3>(s, a, b, work, count, st);
         default: return launch_k1w<LOGR>(s, a, b, work, count, st, poly_only);
     }
 }
