@@ -2,8 +2,8 @@
 
 The library's kernels may start while the kernel before them on the stream still runs and then wait
 for it: behind a caller's kernel that lets its dependents start at once and outlasts the limit of
-the kernels' bounded waits (1 s), and in captured graphs, whose buffers later calls must leave
-alone.  Against the oracle."""
+the kernels' bounded waits (1 s), in chains of products that feed one another, and in captured graphs,
+whose buffers later calls must leave alone.  Against the oracle."""
 import numpy as np
 import pytest
 
@@ -88,3 +88,57 @@ def test_captured_batches_keep_the_plans_workspace(cuda):
             torch.cuda.synchronize()
             got = c.cpu().numpy().view(np.uint64)
             assert all((got[k] == want[pick[k][0]][pick[k][1]]).all() for k in range(len(c)))
+
+
+@pytest.mark.parametrize("n,bits,limbs,count", [
+    (128, 300, 6, 2), (256, 868, 14, 1), (1024, 517, 9, 1), (4096, 868, 14, 2), (4096, 517, 9, 12),
+    (1024, 868, 14, 40), (1024, 190, 3, 40), (16384, 400, 8, 1)])
+def test_products_that_feed_one_another(cuda, n, bits, limbs, count):
+    """Each product reads what the one before wrote, over two plans that share a workspace, with copies
+    and another stream's work in between and no synchronisation; then the same captured."""
+    torch = cuda
+    rng = np.random.default_rng(n + bits + count)
+    q = random_q(rng, bits)
+    first = [uniform_below(rng, q, n, limbs) for _ in range(2)]
+    a, b = (torch.from_numpy(np.stack([x] * count).view(np.int64)).cuda() for x in first)
+    c, d = torch.zeros_like(a), torch.zeros_like(a)
+    steps = 4
+    side = torch.cuda.Stream()
+    with polymul.Plan(n, q, limbs) as p1, polymul.Plan(n, q, limbs) as p2:
+        ws = torch.zeros(p1.workspace_bytes * count, dtype=torch.uint8, device="cuda")
+
+        def multiply(p, x, y, z):
+            p.multiply_batch(x.data_ptr(), y.data_ptr(), z.data_ptr(), count, ws.data_ptr(), ws.numel(),
+                             stream=torch.cuda.current_stream().cuda_stream)
+
+        def chain(delay):
+            x, y = a.clone(), b.clone()
+            for _ in range(steps):
+                multiply(p1, x, y, c)
+                multiply(p2, c, x, d)
+                here = torch.cuda.current_stream()
+                side.wait_stream(here)
+                with torch.cuda.stream(side):
+                    if delay:
+                        torch.cuda._sleep(200000)
+                    x.copy_(d)
+                here.wait_stream(side)
+                multiply(p2, x, c, y)
+            return y
+
+        x, y = first
+        for _ in range(steps):
+            u = oracle.rns_multiply(x, y, q)
+            x = oracle.rns_multiply(u, x, q)
+            y = oracle.rns_multiply(x, u, q)
+        for delay in (False, True):
+            got = chain(delay).cpu().numpy().view(np.uint64)
+            assert (got[0] == y).all() and (got[-1] == y).all()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = chain(False)
+        for _ in range(2):
+            c.zero_()
+            graph.replay()
+            got = out.cpu().numpy().view(np.uint64)
+            assert (got[0] == y).all() and (got[-1] == y).all()
