@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
     constexpr int COLS = 8 * F, HALF = 4 * F;    // a tile's columns, a warp's
     constexpr int SPAN = 256 >> LOGF;            // bytes of a coefficient in K
     constexpr int BOX = 128 * SPAN;              // one row block of a tile
+    constexpr bool kDependent = std::is_same<Work, PlanFoldWork>::value;  // a plan's launch is a programmatic dependent
     constexpr int LOGJ = 4 - LOGF, NTW = J - 1;  // the remaining stages and their twiddles per lane
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* sbase = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
             reinterpret_cast<uint4*>(sX)[k] = make_uint4(0, 0, 0, 0);
     if (warp == 0) {
         tc::tmem_alloc(&tmem_base, 512);
-        grid_trigger();
+        if (kDependent) grid_trigger();
     }
     auto issue = [&](int kk) {
         const TileItem it = w.item(begin + kk);
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
     // products at n = 32768.  Rows without tensor maps: the warps that load wait below, all others meet
     // them at a barrier (60 products of 517 bits at n = 4096, whole: 125.6 us with no wait, 126.4 with a
     // wait in each branch, 124.7 so).
-    if (!PLAIN) {
+    if (!PLAIN && kDependent) {
         grid_wait();
         if (tid == 32 * 4 * kFoldSets)
             for (int kk = 0; kk < kFoldTiles && kk < tiles; ++kk) issue(kk);
@@ -202,7 +203,11 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
         int issued = 0, seen = 0, committed = 0;  // tiles requested, seen complete, given to the tensor cores
         bool w_pending = false;
         if (tiles > 0) {
-            if (!PLAIN) issued = min(kFoldTiles, tiles);
+            if (!PLAIN && kDependent)
+                issued = min(kFoldTiles, tiles);
+            else if (!PLAIN)
+                for (; issued < kFoldTiles && issued < tiles; ++issued)
+                    if (lane == 0) issue(issued);
             w_pending = !wait(&w_full, 0);
         }
         for (int kk = 0; kk < tiles && ok; ++kk) {
