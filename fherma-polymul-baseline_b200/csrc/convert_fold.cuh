@@ -26,14 +26,14 @@
 // and MMAs (a warp of its own for the loads measured 5% slower); kFoldSets sets of four warps (the 128 TMEM lanes) take half tiles (half the columns)
 // in turn, so one set's stages and stores overlap another's accumulator reads.
 // Measured: 6.98 -> 5.60 us a product (868 bits, n = 32768, 128 products), 3.13 -> 2.72 us at
-// n = 16384 (640 bits), 2.05 -> 1.53 us at n = 8192.  At 32768 it issues 21 instructions a residue
-// (K1W 30) and moves 22.8 MB in 5.6 us (4.1 TB/s); left are the multiply pipe (62%), the 32-byte
-// stores (each touches its own line: 32 lines an instruction; 16-byte ones cost 0.2 ms more) and
-// the chain MMA - accumulator read - stages of few warps (three sets of 128 registers; two
-// of 168 and four of 96 measured 1-2% and 23% slower).  The form without tensor maps converts 60
-// products of 517 bits (9 limbs, n = 4096) in 64 us against 54 for the same with 10 limbs by TMA
-// (one loader warp 99, two 70); copying rows of even limbs 16 bytes at a time instead of by
-// TMA measured 6% to 13% slower.
+// n = 16384 (640 bits), 2.05 -> 1.53 us at n = 8192; 5.35 - 5.6 us at 32768 by box.  There it
+// issues 24 instructions a residue (K1W 30) and moves 22.8 MB in 5.5 us (4.1 TB/s); left are
+// the multiply pipe (busy 61% of its cycles), the 32-byte stores (each touches its own line: 29.5
+// sectors an instruction; 16-byte ones cost 0.2 ms more) and the chain MMA - accumulator read -
+// stages of few warps (three sets of 128 registers; two of 168 and four of 96 measured 1-2%
+// and 23% slower).  The form without tensor maps converts 60 products of 517 bits (9 limbs,
+// n = 4096) in 58 us against 47 for the same with 10 limbs by TMA (one loader warp 99, two 70);
+// copying rows of even limbs 16 bytes at a time instead of by TMA measured 6% to 13% slower.
 // Barriers: tma_full[3]; full[set][pair] (an accumulator pair is complete) and done[3] (the
 // tile's buffer is free), from MMA commits; empty[pair] (one arrival a warp: the pair has been
 // read); w_full.  Every wait is bounded; one that gives up stops the CTA, lets its

@@ -9,7 +9,7 @@
 //   c_m = (1/4) r_i^-m sum_j iota_i^-jm C_ij   (mod p_i),
 // a 4-point inverse DFT (one butterfly level across thread pairs by warp
 // shuffle, one in registers) and a scale that also carries the CRT factor
-// s_i = 2^32 n^-1 (P/p_i)^-1.  One INT8 contraction then gives
+// s_i = 2^32 (n/4)^-1 (P/p_i)^-1 (the rows' transforms stop two stages short).  One INT8 contraction then gives
 //   c = sum_m 2^(bbits m) (sum_i t_mi (P/p_i) - k_m P)  mod q,
 // with K = 4 components x 16 primes x 4 bytes = 256 and N = 160 columns: the
 // value bytes of sum t_mi ((P/p_i) 2^(bbits m) mod q) (4W + 4 of them) and, per

@@ -108,7 +108,8 @@ void* fherma_init(const fherma::Point& p) {
     s->n = p.N;
     s->words = p.L;
     const uint32_t limbs = p.L / 2;
-    // the tensor-core conversion reads 16-byte coefficient rows (even limb counts)
+    // an odd limb count has no 16-byte coefficient rows, which PM_CONVERT_TENSOR asks for: the default path
+    // (the tensor cores all the same from n = 256 on)
     const uint32_t flags = (limbs % 2 == 0) ? PM_CONVERT_TENSOR : PM_CONVERT_DEFAULT;
     const int st = pm_plan_create(&s->plan, p.N, q64.data(), limbs, limbs, flags);
     if (st != PM_OK) raise(st, "fherma_init");

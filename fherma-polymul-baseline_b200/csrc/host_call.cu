@@ -142,10 +142,11 @@ struct CopyJob {
 // too.  Idle workers spin for a while (back-to-back calls find them awake), then sleep on
 // a condition variable.  Every plan of the process shares one pool, made with the first
 // plan that needs it and ended with the last: a pool per plan left each plan's threads
-// spinning through the other plans' calls (three plans called in turn on a 16-vCPU host took
-// 1010 us a call at N = 32768 against 350 alone; 345 with the shared pool).  Jobs of calls on several
-// threads are open side by side; workers never wait inside a piece, so one call's
-// pending pieces do not hold up another's.
+// spinning through the other plans' calls, and threads that call at once had eight each to share the
+// cores.  N = 32768 on a 16-vCPU host, us a product, a pool per plan / one pool: calls from one thread
+// 361 / 353 (three plans in turn 345 / 331), from two with a plan each 317 / 218, from four 482 / 195, from
+// eight 739 / 196.  Jobs of calls on several threads are open side by side; workers never wait
+// inside a piece, so one call's pending pieces do not hold up another's.
 class CopyPool {
 public:
     explicit CopyPool(int threads) {

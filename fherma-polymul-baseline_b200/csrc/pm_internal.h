@@ -105,7 +105,8 @@ struct HostCall {
     ~HostCall();
 };
 
-// Largest launch group by default, and the largest a caller may set.
+// Largest launch group by default (of small products, see default_group, more), and the largest a caller
+// may set.
 constexpr uint32_t kMaxDefaultGroup = 128;
 constexpr size_t kSmallGroupBytes = size_t(64) << 20;  // residue planes up to which a default group may pass that,
 constexpr uint32_t kMaxSmallGroup = 4096;              // up to this many products (grid dimensions)
@@ -118,7 +119,7 @@ struct Tuning {
     int crt_ctas_per_sm = 0;   // K3T persistent CTAs per SM; 0: as many as fit (k3t_ctas_per_sm)
     bool row_persistent = true;  // K2P (rows of C >= 1024) and K2W (16 .. 512) instead of K2
     bool conv_whole_basis = true;  // tensor conversion: one pass of a tile over every prime (K1W) or per group (K1T)
-    uint32_t group = 0;        // products per launch group in batches (0: up to ~2 GB of residues, <= 128)
+    uint32_t group = 0;        // products per launch group in batches (0: default_group)
     bool tuned = false;
 };
 

@@ -299,7 +299,7 @@ void PlanCore::init(uint32_t n_, const uint64_t* q64, uint32_t q_limbs, uint32_t
         throw Failure(PM_ERR_INVALID, "PM_CONVERT_TENSOR and PM_CONVERT_SIMT exclude each other");
     // No path asked for: the tensor path, over an odd coef_limbs (row pitches a tensor map cannot
     // describe) by the conversion kernels' plain-row forms, which take rows of 16 columns or more
-    // (n >= 256).  60 products of 517 bits (9 limbs) at n = 4096: 396 us by the plain method, 135 us so.
+    // (n >= 256).  60 products of 517 bits (9 limbs) at n = 4096: 392 us by the plain method, 124 us so.
     plain_rows = false;
     if (!(flags_ & (PM_CONVERT_TENSOR | PM_CONVERT_SIMT | PM_WIDE_NTT)) &&
         (coef_limbs_ % 2 == 0 || (n_ >= 256 && !(flags_ & PM_QUARTIC)))) {
@@ -656,7 +656,8 @@ void check_device_errors(const PlanCore& s) {
 // faster than 128), and the row kernel's DRAM traffic stays at its algorithmic
 // bytes.  Products of few residues go in larger groups, as many as keep their planes at 64 MB
 // (half the L2): a launch of 128 of them is mostly its own start and end.  500 products of 200
-// bits at n = 1024 (57 MB): 158 us in four groups of at most 128, 92 us in one.
+// bits at n = 1024 (57 MB): 116 us in four groups of at most 128, 75.5 in one; 600 (68 MB) 142 us in
+// five, 98.7 in the two that the line leaves.
 uint32_t default_group(const PlanCore& s) {
     const size_t budget = size_t(2) << 30;
     size_t g = budget / s.workspace_bytes;

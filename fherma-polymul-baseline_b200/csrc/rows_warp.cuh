@@ -13,11 +13,12 @@
 // Here 16 values a lane leave one exchange (two at C = 512), with 16-byte shared accesses on
 // the closing side.
 //
-// Measured (868-bit q unless said): 250 -> 236 us for 100 products at n = 8192 (C = 512), 62 ->
-// 41 us for 60 of 517 bits at n = 4096 on the plain path (C = 128), 82 -> 59 us for 500 of 200 bits at
-// n = 1024 (C = 64).  It runs the multiply pipe 64% of the time (a lazy butterfly, 8 pipe
-// cycles, takes 9.2 in a loop of nothing else at 4 warps a sub-partition); 4 and 6 CTAs per
-// SM instead of 5 measured within 2% of it either way.
+// Measured in the same launches, k2_rows / this kernel (868-bit q unless said): 100 products at
+// n = 8192 (C = 512) 247 / 235 us, 500 of 200 bits at n = 1024 (C = 64) 43.5 / 31.4, 60 of 517 bits at
+// n = 4096 (C = 256) 47.1 / 47.0, and 130.2 / 124.7 for that whole call, as k2_rows is no dependent
+// launch.  It runs the multiply pipe 66% of the time (a lazy butterfly, 8 pipe cycles, takes 9.2 in
+// a loop of nothing else at 4 warps a sub-partition); 4 and 6 CTAs per SM instead of 5 measured
+// within 2% of it either way.
 //
 // Layouts of a row of C values over T = C/16 lanes (t = lane % T):
 //   first    value l*G + m of lane t is word t*G + m + D*l   (D = 16, or 32 at C = 512; G = D/T):

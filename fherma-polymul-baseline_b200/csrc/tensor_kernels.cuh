@@ -432,7 +432,7 @@ __device__ __forceinline__ void add1_carry(uint32_t& a, uint32_t b, uint32_t& cy
 // Primes a tile holds: W <= 12 words (q of up to 384 bits) need at most 27, so those kernels take
 // boxes, digit tiles and weights of 32 instead of 64 (52 KB a CTA instead of 104) and only the K
 // steps the primes fill; three CTAs share an SM.  Measured for 500 products of 200 bits at n = 1024:
-// 37.2 -> 31.3 us; an uneven batch of 200 to 868 bits, whole, 401 -> 390.
+// 37.2 -> 31.3 us (with two CTAs an SM 33.5); an uneven batch of 200 to 868 bits, whole, 401 -> 390.
 constexpr int crt_cap(int W) { return W <= 12 ? 32 : 64; }
 constexpr int k3t_min_blocks(int W) { return W <= 12 ? 3 : 2; }
 

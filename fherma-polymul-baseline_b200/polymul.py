@@ -166,7 +166,7 @@ class Plan:
     """A product plan for (n, q): basis, CRT constants, workspace, staging."""
 
     def __init__(self, n, q, coef_limbs=None, tensor=None, special_form=False, wide=False, quartic=False):
-        """tensor: None lets the library choose (the tensor path when coef_limbs is even),
+        """tensor: None lets the library choose (the tensor path when coef_limbs is even or n >= 256),
         True asks for the tcgen05 conversion/CRT, False for the plain method."""
         self.q = int(q)
         qarr = q_limbs_of(self.q)

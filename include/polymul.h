@@ -215,8 +215,8 @@ int pm_basis_query(uint32_t n, uint32_t q_bits, uint32_t* primes, uint32_t capac
 /* ------------------------------------------------------------------------
  * Uneven batches: `count` products of different n (256..65536) and different
  * odd q, all on the tensor path, run as one CUDA graph of persistent kernels
- * over flat work tables (conversion items ordered by prime group, row items per
- * ring size, CRT items per width).  The batch owns packed device buffers:
+ * over flat work tables (conversion items per class of basis, in small batches
+ * by prime group; row items per ring size, CRT items per width).  The batch owns packed device buffers:
  * product z's a, b, c start offsets[z] u64 words into the buffers returned by
  * pm_batch_buffers, each n_z x coef_limbs.  No counterpart in the reference.
  * ------------------------------------------------------------------------ */
