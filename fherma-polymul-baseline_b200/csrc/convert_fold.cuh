@@ -126,6 +126,10 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
     constexpr int BOX = 128 * SPAN;              // one row block of a tile
     constexpr bool kDependent = std::is_same<Work, PlanFoldWork>::value;  // a plan's launch is a programmatic dependent
     constexpr int LOGJ = 4 - LOGF, NTW = J - 1;  // the remaining stages and their twiddles per lane
+    // Tiles requested before the CTA's first barrier, where the other threads wait for the one that requests
+    // a tile's 2^f copies: all three at f = 1, else one (500 products of 200 bits at n = 1024, whole, three /
+    // one: 75.6 / 75.0 us).
+    constexpr int FIRST = LOGF == 1 ? kFoldTiles : 1;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* sbase = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sW = sbase;                     // [4][2][128 rows x 128 B]
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
     if (!PLAIN && kDependent) {
         grid_wait();
         if (tid == 32 * 4 * kFoldSets)
-            for (int kk = 0; kk < kFoldTiles && kk < tiles; ++kk) issue(kk);
+            for (int kk = 0; kk < FIRST && kk < tiles; ++kk) issue(kk);
     }
     tc::fence_smem_async();
     tc::fence_before();
@@ -203,9 +207,8 @@ __global__ void __launch_bounds__(k1f_threads(PLAIN), 1)
         int issued = 0, seen = 0, committed = 0;  // tiles requested, seen complete, given to the tensor cores
         bool w_pending = false;
         if (tiles > 0) {
-            if (!PLAIN && kDependent)
-                issued = min(kFoldTiles, tiles);
-            else if (!PLAIN)
+            if (!PLAIN && kDependent) issued = min(FIRST, tiles);
+            if (!PLAIN && (!kDependent || FIRST < kFoldTiles))
                 for (; issued < kFoldTiles && issued < tiles; ++issued)
                     if (lane == 0) issue(issued);
             w_pending = !wait(&w_full, 0);
